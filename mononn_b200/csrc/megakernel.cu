@@ -63,6 +63,19 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
       : "memory");
   return ok;
 }
+// The same test without the bounded suspension of the thread: a look ahead that must not hold up
+// the instructions behind it.
+__device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int32_t x, int32_t y,
                                             uint32_t bar) {
   asm volatile(
@@ -119,6 +132,39 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+// Upper half of every operand descriptor (see umma_desc_sw128): 8-row groups 1024 B apart, version 1,
+// 128-byte swizzle. The lower half holds the start address in 16-byte units and the leading offset.
+constexpr uint32_t kDescHi = 64u | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+// One 64-wide k block: four MMAs (K = 16 each, 32 bytes further along both operands' rows), then the
+// commit that frees the activation slot and, for the last k block of a weight slot, the one that
+// frees that slot. One block of straight-line predicated code: the loop around it is bound by the
+// number of instructions that its single warp issues. With a branch around each instruction and the
+// descriptors assembled in 64 bits a k block of a 64-column tile took 0.30 us, this way 0.20; see
+// also the loop in role_mma.
+__device__ __forceinline__ void mma_kblock(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                           uint32_t accumulate, uint32_t a_empty, uint32_t b_empty, bool free_b) {
+  asm volatile(
+      "{\n\t.reg .pred q, p, f, w;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t.reg .b32 t;\n\t"
+      "setp.eq.u32 w, 0, 0;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.u32 p, %4, 0;\n\t"
+      "setp.ne.and.u32 f, %7, 0, q;\n\t"
+      "mov.b64 a0, {%1, %8};\n\tmov.b64 b0, {%2, %8};\n\t"
+      "add.u32 t, %1, 2;\n\tmov.b64 a1, {t, %8};\n\tadd.u32 t, %2, 2;\n\tmov.b64 b1, {t, %8};\n\t"
+      "add.u32 t, %1, 4;\n\tmov.b64 a2, {t, %8};\n\tadd.u32 t, %2, 4;\n\tmov.b64 b2, {t, %8};\n\t"
+      "add.u32 t, %1, 6;\n\tmov.b64 a3, {t, %8};\n\tadd.u32 t, %2, 6;\n\tmov.b64 b3, {t, %8};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b0, %3, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, w;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, w;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, w;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "@f tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
+      "}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(a_empty), "r"(b_empty),
+      "r"(static_cast<uint32_t>(free_b)), "r"(kDescHi)
       : "memory");
 }
 // One lane of a converged warp (the same one every time for a full mask).
@@ -352,14 +398,16 @@ __device__ __forceinline__ void trace(const KernelParams& P, uint32_t stage, uin
 // path is out of line so that the many wait sites stay a few instructions each.
 __device__ __noinline__ bool mbar_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t b,
                                             uint32_t parity, uint32_t stage, uint32_t where) {
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
   const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
   uint32_t it = 0;
   for (;;) {
     if (mbar_try_wait(b, parity)) return true;
     if ((++it & 63u) == 0u) {
       if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit) {
         report_failure(P, ctrl, stage, ST_MBARRIER_TIMEOUT, where);
         return false;
       }
@@ -414,7 +462,7 @@ __device__ __forceinline__ void acquire_after_poll(const uint32_t* p) {
 // instead of 1300.
 __device__ __noinline__ bool grid_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t target,
                                             uint32_t stage, uint32_t where) {
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
   const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
   uint32_t it = 0;
   for (;;) {
@@ -431,7 +479,9 @@ __device__ __noinline__ bool grid_wait_slow(const KernelParams* P, Ctrl* ctrl, u
         *reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit) {
         report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
         return false;
       }
@@ -457,14 +507,16 @@ __device__ __forceinline__ bool grid_wait(const Ctx& c, uint32_t stage, uint32_t
 // poller's acquire at GPU scope orders the other CTAs' stores before this thread's loads).
 __device__ __noinline__ bool local_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t need,
                                              uint32_t stage, uint32_t where) {
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
   const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
   uint32_t it = 0;
   for (;;) {
     if (ld_acquire_cta_smem(&ctrl->barriers_seen) >= need) return true;
     if ((++it & 63u) == 0u) {
       if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit) {
         report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
         return false;
       }
@@ -503,7 +555,7 @@ __device__ __forceinline__ bool grid_wait_warp(const Ctx& c, uint32_t stage, uin
 // never depend on a waiter.
 __device__ __noinline__ bool flag_wait_slow(const KernelParams* P, Ctrl* ctrl, const uint32_t* flag,
                                             uint32_t target, uint32_t stage, uint32_t where) {
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
   const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
   uint32_t it = 0;
   for (;;) {
@@ -517,7 +569,9 @@ __device__ __noinline__ bool flag_wait_slow(const KernelParams* P, Ctrl* ctrl, c
         *reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit) {
         report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
         return false;
       }
@@ -881,6 +935,43 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
   }
 }
 
+// The MMA issuer's place in the two rings, kept as slot and parity (a count would be divided by the
+// number of slots on every k block) with the shared-memory addresses worked out once.
+struct MmaRing {
+  uint32_t a_slot = 0, a_par = 0, b_slot = 0, b_par = 0;
+  uint32_t a_full0, a_empty0, b_full0, b_empty0, a_lo0, b_lo0;
+  __device__ __forceinline__ explicit MmaRing(const Ctx& c)
+      : a_full0(smem_u32(&c.ctrl->a_full[0])), a_empty0(smem_u32(&c.ctrl->a_empty[0])),
+        b_full0(smem_u32(&c.ctrl->b_full[0])), b_empty0(smem_u32(&c.ctrl->b_empty[0])),
+        a_lo0(umma_desc_lo(c.a_ring)), b_lo0(umma_desc_lo(c.b_ring)) {}
+  __device__ __forceinline__ uint32_t a_lo() const { return a_lo0 + a_slot * (kSlotBytes >> 4); }
+  __device__ __forceinline__ uint32_t b_lo() const { return b_lo0 + b_slot * (kBSlotBytes >> 4); }
+  __device__ __forceinline__ uint32_t a_empty() const { return a_empty0 + a_slot * 8u; }
+  __device__ __forceinline__ uint32_t b_empty() const { return b_empty0 + b_slot * 8u; }
+  __device__ __forceinline__ uint32_t a_peek() const { return mbar_test_wait(a_full0 + a_slot * 8u, a_par); }
+  __device__ __forceinline__ uint32_t b_peek() const { return mbar_test_wait(b_full0 + b_slot * 8u, b_par); }
+  __device__ __forceinline__ bool a_wait(const Ctx& c, uint32_t where) const {
+    const uint32_t bar = a_full0 + a_slot * 8u;
+    return mbar_try_wait(bar, a_par) || mbar_wait_slow(c.P, c.ctrl, bar, a_par, c.stage, where);
+  }
+  __device__ __forceinline__ bool b_wait(const Ctx& c, uint32_t where) const {
+    const uint32_t bar = b_full0 + b_slot * 8u;
+    return mbar_try_wait(bar, b_par) || mbar_wait_slow(c.P, c.ctrl, bar, b_par, c.stage, where);
+  }
+  __device__ __forceinline__ void a_next() {
+    if (++a_slot == kASlots) { a_slot = 0; a_par ^= 1u; }
+  }
+  __device__ __forceinline__ void b_next() {
+    if (++b_slot == kBSlots) { b_slot = 0; b_par ^= 1u; }
+  }
+  // activation slots used so far modulo two rounds: what the attention code counts slots from
+  __device__ __forceinline__ uint32_t a_count() const { return a_par * kASlots + a_slot; }
+  __device__ __forceinline__ void a_set(uint32_t count) {
+    a_slot = count % kASlots;
+    a_par = (count / kASlots) & 1u;
+  }
+};
+
 // ----------------------------------------------------------------------------
 // Role: MMA issuer (warp 2). All 32 lanes run the loop converged and one elected lane issues the
 // tcgen05 instructions: the operands of a converged warp can be kept in uniform registers, and
@@ -890,7 +981,8 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
 __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
   const KernelParams& P = *c.P;
   const bool issuer = elect_one_sync();
-  uint32_t a_cnt = 0, b_cnt = 0, acc_cnt = 0;
+  MmaRing ring(c);
+  uint32_t acc_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
     const StageDesc st = load_stage(P, s);
@@ -904,38 +996,38 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * kAccCols;
         const uint32_t idesc = umma_idesc_m128(op.n_tile);
-        uint32_t b_slot = 0;
-        for (uint32_t kb = 0, next_sub = 0; kb < nkb; ++kb) {
-          const uint32_t sub = next_sub;  // kb % kbps without the division (this loop is bound by its issue path)
-          next_sub = (sub + 1u == kbps) ? 0u : sub + 1u;
+        const uint32_t sub_step = op.n_tile * 8u;  // one k block further in a weight slot, in 16-byte units
+        uint32_t sub = 0, b_lo = 0;
+        uint32_t a_rdy = ring.a_peek(), b_rdy = ring.b_peek();
+        for (uint32_t kb = 0; kb < nkb; ++kb) {
           if (sub == 0) {
-            b_slot = b_cnt % kBSlots;
-            WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->b_full[b_slot], (b_cnt / kBSlots) & 1u, 0x301));
+            if (!b_rdy) WAIT_OR_RETURN(ring.b_wait(c, 0x301));
+            b_lo = ring.b_lo();
           }
-          const uint32_t a_slot = a_cnt % kASlots;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[a_slot], (a_cnt / kASlots) & 1u, 0x302));
+          if (!a_rdy) WAIT_OR_RETURN(ring.a_wait(c, 0x302));
           if (kb == 0) if (issuer) trace(P, s, TR_MMA_FIRST);
-          tc_fence_after();
-          const uint64_t ad = umma_desc_sw128(c.a_ring + a_slot * kSlotBytes);
-          const uint64_t bd =
-              umma_desc_sw128(c.b_ring + b_slot * kBSlotBytes + sub * op.n_tile * 128u);
-#pragma unroll
-          for (uint32_t k = 0; k < 4; ++k)
-            if (issuer) tc_mma_f16(tmem_d, ad + 2u * k, bd + 2u * k, idesc, (kb | k) != 0u);
-          if (issuer) tc_commit(smem_u32(&c.ctrl->a_empty[a_slot]));
-          ++a_cnt;
-          if (sub + 1 == kbps || kb + 1 == nkb) {
-            if (issuer) tc_commit(smem_u32(&c.ctrl->b_empty[b_slot]));
-            ++b_cnt;
+          const uint32_t a_lo = ring.a_lo(), a_empty = ring.a_empty(), b_empty = ring.b_empty();
+          const bool last_sub = (++sub == kbps) || kb + 1u == nkb;
+          ring.a_next();
+          if (last_sub) {
+            sub = 0;
+            ring.b_next();
           }
+          // the next k block's barriers are tested before this one's instructions go out, so that
+          // the tests' latency passes while the tensor core works
+          a_rdy = ring.a_peek();
+          b_rdy = ring.b_peek();
+          tc_fence_after();
+          mma_kblock(tmem_d, a_lo, b_lo, idesc, kb, a_empty, b_empty, last_sub);
+          b_lo += sub_step;
         }
         if (issuer) tc_commit(smem_u32(&c.ctrl->acc_full[buf]));
         ++acc_cnt;
         if (issuer) trace(P, s, TR_MMA_LAST);
       } else if (op.kind == OP_ATTENTION) {
         const uint32_t nc = attn_chunks(op);
-        uint32_t base = a_cnt, ph = acc_cnt;
-        a_cnt += attn_slots(op);
+        uint32_t base = ring.a_count(), ph = acc_cnt;
+        const uint32_t after = base + attn_slots(op);
         auto slot_of = [](uint32_t cnt) { return cnt % kASlots; };
         auto par_of = [](uint32_t cnt) { return (cnt / kASlots) & 1u; };
         if (attn_fused(op)) {
@@ -945,20 +1037,18 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
           WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[ph & 1u], ((ph >> 1) & 1u) ^ 1u, 0x321));
           tc_fence_after();
           const uint32_t idesc = umma_idesc_m128(192);
+          uint32_t a_rdy = ring.a_peek(), b_rdy = ring.b_peek();
           for (uint32_t kb = 0; kb < nkb; ++kb) {
-            const uint32_t b_slot = b_cnt % kBSlots, a_c = base + kb;
-            WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->b_full[b_slot], (b_cnt / kBSlots) & 1u, 0x322));
-            WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(a_c)], par_of(a_c), 0x323));
+            if (!b_rdy) WAIT_OR_RETURN(ring.b_wait(c, 0x322));
+            if (!a_rdy) WAIT_OR_RETURN(ring.a_wait(c, 0x323));
             if (kb == 0) if (issuer) trace(P, s, TR_MMA_FIRST);
+            const uint32_t a_lo = ring.a_lo(), b_lo = ring.b_lo(), a_empty = ring.a_empty(), b_empty = ring.b_empty();
+            ring.a_next();
+            ring.b_next();
+            a_rdy = ring.a_peek();
+            b_rdy = ring.b_peek();
             tc_fence_after();
-            const uint64_t ad = umma_desc_sw128(c.a_ring + slot_of(a_c) * kSlotBytes);
-            const uint64_t bd = umma_desc_sw128(c.b_ring + b_slot * kBSlotBytes);
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)
-              if (issuer) tc_mma_f16(tmem_base + kAttnQkvCol, ad + 2u * k, bd + 2u * k, idesc, (kb | k) != 0u);
-            if (issuer) tc_commit(smem_u32(&c.ctrl->a_empty[slot_of(a_c)]));
-            if (issuer) tc_commit(smem_u32(&c.ctrl->b_empty[b_slot]));
-            ++b_cnt;
+            mma_kblock(tmem_base + kAttnQkvCol, a_lo, b_lo, idesc, kb, a_empty, b_empty, true);
           }
           if (issuer) tc_commit(smem_u32(&c.ctrl->acc_full[phQ & 1u]));
           if (issuer) trace(P, s, TR_MMA_LAST);
@@ -1004,6 +1094,7 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         }
         if (issuer) tc_commit(smem_u32(&c.ctrl->acc_full[phO & 1u]));
         acc_cnt = ph + 2u;
+        ring.a_set(after);
       }
     }
   }
