@@ -189,7 +189,7 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-// Issue only: the registers are valid after the next tc_wait_ld(). Lets the following load be in
+// Issue only: the registers are valid after tc_wait_ld on them. Lets the following load be in
 // flight while the previous one is processed.
 __device__ __forceinline__ void tc_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
   __syncwarp();
@@ -205,8 +205,17 @@ __device__ __forceinline__ void tc_ld32_issue(uint32_t taddr, uint32_t (&r)[32])
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tc_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// The wait names the registers of a load issued before it, so that nothing that uses them moves ahead.
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+                 "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]),
+                 "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]),
+                 "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
+                 "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]),
+                 "+r"(r[31])
+               :
+               : "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -332,12 +341,13 @@ struct Ctrl {
   float mask_row[384];      // additive key mask of the current attention tile (log2 units)
   float row_max[2][128];    // attention: row maximum / row sum over each warp half's columns,
   float row_sum[2][128];    // exchanged between the two threads that share a query row
-  float ln_part[2][kSplitRowsPerItem][4];  // split LayerNorm: per-warp partial sum / squared deviation
+  float2 ln_part[2][kSimtWarps];  // LayerNorm rows shared by several warps: per-warp (sum, squared deviations)
   float red_val[kSimtWarps];  // arg-max: per-warp partial results of the current row
   uint32_t red_idx[kSimtWarps];
   // Shared-memory copies of the operator descriptor each role is working on: slot 0 weight
   // producer, 1 activation producer, 2 MMA issuer, 3.. the eight epilogue warps.
   uint4 desc[3 + kSimtWarps][16];
+  uint4 stage_desc[3 + kSimtWarps][3];
 };
 
 static_assert(sizeof(Ctrl) <= kCtrlBytes, "control block exceeds its shared-memory reserve");
@@ -625,14 +635,15 @@ struct Item {
 // Descriptors are read with straight-line code (no branch between two loads, which would
 // serialise them) into registers / shared memory, and the first item's descriptor of a stage
 // is fetched before the role waits for the previous stage's barrier.
-__device__ __forceinline__ StageDesc load_stage(const KernelParams& P, uint32_t s) {
-  StageDesc st;
-  const uint4* g = reinterpret_cast<const uint4*>(P.stages + s);
-  uint4* d = reinterpret_cast<uint4*>(&st);
-  d[0] = __ldg(g);
-  d[1] = __ldg(g + 1);
-  d[2] = __ldg(g + 2);
-  return st;
+// The stage descriptor goes to the role's slot in shared memory: kept in registers, its item ranges
+// would be live across all of a stage's work.
+__device__ __forceinline__ const StageDesc& load_stage(const KernelParams& P, Ctrl* ctrl, uint32_t role, uint32_t s,
+                                                       uint32_t lane) {
+  uint4* slot = ctrl->stage_desc[role];
+  __syncwarp();
+  if (lane < sizeof(StageDesc) / 16u) slot[lane] = __ldg(reinterpret_cast<const uint4*>(P.stages + s) + lane);
+  __syncwarp();
+  return *reinterpret_cast<const StageDesc*>(slot);
 }
 
 // Copies the descriptor of the operator that owns work item `item` of the stage into `slot`
@@ -738,7 +749,7 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
   uint32_t b_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
-    const StageDesc st = load_stage(P, s);
+    const StageDesc& st = load_stage(P, c.ctrl, 0u, s, lane);
     {
       // If the stage holds attention items that compute their own projections, only a few SMs will
       // pull those weights, each through a three-slot ring. The CTAs that got none of those items
@@ -823,7 +834,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
   uint32_t a_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
-    const StageDesc st = load_stage(P, s);
+    const StageDesc& st = load_stage(P, c.ctrl, 1u, s, lane);
     Item first{nullptr, 0};
     if (blockIdx.x < st.n_items) {
       first = fetch_item<true>(P, st, blockIdx.x, c.ctrl->desc[1], lane);
@@ -985,7 +996,7 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
   uint32_t acc_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
-    const StageDesc st = load_stage(P, s);
+    const StageDesc& st = load_stage(P, c.ctrl, 2u, s, lane);
     for (uint32_t item = blockIdx.x; item < st.n_items; item += gridDim.x) {
       const Item it = fetch_item<true>(P, st, item, c.ctrl->desc[2], lane);
       const OpDesc& op = *it.op;
@@ -1187,7 +1198,7 @@ __device__ __forceinline__ void add4(float4& a, const float4 b) {
 // Accumulator row `quarter * 32 + lane` (TMEM lane = row) is shared by the two warps of the
 // quarter: warp `half` takes every other column group of the tile (groups of 32 columns, of 16
 // for tiles up to 32 wide so that both warps have work).
-__device__ __noinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t, uint32_t tmem_acc,
+__device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t, uint32_t tmem_acc,
                                            uint32_t quarter, uint32_t half, uint32_t lane,
                                            const float* bias_s, uint8_t* stg) {
   const uint32_t grow = t.mt * 128u + quarter * 32u + lane;
@@ -1347,7 +1358,7 @@ __device__ __forceinline__ void row_emit(float4 a, float mean, float rstd, uint3
 
 // LayerNorm / embedding item: eight rows, one warp each. Rows up to 1024 columns stay in
 // registers between the statistics and the normalisation; wider rows are re-read.
-__device__ __noinline__ void rowwise_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
+__device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
                                           uint32_t lane, const KernelParams& P, uint32_t stage) {
   const uint32_t row = local * kRowsPerItem + warp_in_group;
   if (row >= op.rows) return;
@@ -1569,130 +1580,177 @@ __device__ __forceinline__ void prefetch_row_consts(const OpDesc& op, uint32_t l
   }
 }
 
-// LayerNorm / RMS norm of few rows: four warps share a row (two rows per work item), each
-// taking a quarter of the columns; the partial sums meet in shared memory. With 128 rows this
-// puts 512 warps on 64 SMs instead of 128 warps on 16, and cuts the per-warp chain of loads,
-// reductions, conversions and stores (about 2 us for a 768-column row on one warp) to a quarter.
-__device__ __noinline__ bool rowwise_split_item(Ctx& c, const OpDesc& op, uint32_t local, uint32_t widx,
-                                                uint32_t lane) {
-  const uint32_t r_in = widx >> 2, part = widx & 3u;
-  const uint32_t row = local * kSplitRowsPerItem + r_in;
-  const bool live = row < op.rows;
-  const uint32_t safe_row = live ? row : 0u;
-  const uint32_t cols = op.cols, per = cols >> 4;  // 16-byte f32 vectors per warp (<= 64)
-  const uint32_t flags = op.flags;
-  const bool rms = (flags & F_RMSNORM) != 0u, src32 = (flags & F_SRC_F32) != 0u;
-  const uint32_t v0 = part * per;
-  uint32_t vi[2];
-  bool on[2];
+// LayerNorm / RMS norm / L2 norm over all of this CTA's rows of the operator, `op.row_warps` warps to a
+// row (1, 2 or 4; at most 512 columns a warp, four 16-byte f32 vectors a lane).
+//
+// Bound by latency, not by bytes: a row is a chain of L2 loads, two warp reductions and stores of some
+// 3 us, and with one row per warp and nothing in flight behind it the rows of a large batch took
+// 4 us a wave (6144 rows of 1024: 25 us for 63 MB of L2 traffic), rows of 2048 columns, read three
+// times, four times that. So a warp has two rows in registers: it works on one while the loads of
+// the next are under way. Everything is inline and small enough not to spill: with the counters
+// polled by acquire loads, L1 holds nothing for long and a spilled register is an L2 round trip.
+//
+// The warps that share a row meet once in shared memory with (sum, sum of squared deviations from
+// their own mean), combined pairwise:
+//   M2 = sum_w [ M2_w + n_w (mean_w - mean)^2 ]
+// which is as accurate as the two-pass form. The meeting place is double buffered, so one barrier a
+// row is enough. Returns the number of work items done (local, local + gridDim.x, ..), 0 on abort.
+struct NormRows {
+  const OpDesc& op;
+  uint32_t lane, part, per, v0;  // this warp's part of a row: vectors v0 + 32 i, while lane + 32 i < per
+  uint32_t widx, group, done;    // group: warps per row
+  uint2 gv[4], bv[4], b2v[4];    // scale, shift and pre-load bias of those columns, for all rows
+
+  __device__ __forceinline__ void constants() {
+    const bool plain = (op.flags & F_L2NORM) != 0u, centre = !(op.flags & (F_RMSNORM | F_L2NORM));
+    const bool b2 = op.q[2] != 0 && op.q[3] != 0;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    on[i] = lane + 32u * i < per;
-    vi[i] = v0 + (on[i] ? lane + 32u * i : 0u);
+    for (int i = 0; i < 4; ++i) {
+      gv[i] = make_uint2(0x3c003c00u, 0x3c003c00u);  // 1, 1, 1, 1
+      bv[i] = b2v[i] = make_uint2(0u, 0u);
+      if (lane + 32u * i < per) {
+        if (!plain) gv[i] = __ldg(reinterpret_cast<const uint2*>(op.p[2]) + v0 + 32 * i);
+        if (centre) bv[i] = __ldg(reinterpret_cast<const uint2*>(op.p[3]) + v0 + 32 * i);
+        if (b2) b2v[i] = __ldg(reinterpret_cast<const uint2*>(op.q[3]) + v0 + 32 * i);
+      }
+    }
   }
-  const uint2* gamma = reinterpret_cast<const uint2*>(op.p[2]);
-  const uint2* beta = reinterpret_cast<const uint2*>(op.p[3]);
-  const bool two = op.q[2] != 0, add_b2 = two && op.q[3] != 0;
-  const uint2* b2p = add_b2 ? reinterpret_cast<const uint2*>(op.q[3]) : gamma;
-  uint2 gv[2], bv[2], b2v[2];
-  float4 x[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    gv[i] = __ldg(gamma + vi[i]);
-    bv[i] = __ldg(beta + vi[i]);
-    b2v[i] = __ldg(b2p + vi[i]);
+  // unpacked with each row: kept as f32 they would take twice the registers
+  static __device__ __forceinline__ float4 unpack(uint2 h) {
+    asm volatile("" : "+r"(h.x), "+r"(h.y));
+    return h4_to_f4(h);
   }
-  if (src32) {
-    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(op.p[1]) +
-                                                        static_cast<size_t>(safe_row) * op.lds);
+
+  __device__ __forceinline__ void load(uint32_t row, float4 (&x)[4]) const {
+    if (row >= op.rows) row = 0;
+    if (op.flags & F_SRC_F32) {
+      const float4* p = reinterpret_cast<const float4*>(op.p[1]) + static_cast<size_t>(row) * (op.lds >> 2) + v0;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) x[i] = __ldcg(src + vi[i]);
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) x[i] = __ldcg(p + 32 * i);
+    } else {
+      const uint2* p = reinterpret_cast<const uint2*>(op.p[1]) + static_cast<size_t>(row) * (op.lds >> 2) + v0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) {
+          const uint2 h = __ldcg(p + 32 * i);  // converted when it is used: a conversion here would wait
+          x[i].x = __uint_as_float(h.x);
+          x[i].y = __uint_as_float(h.y);
+        }
+    }
+  }
+  __device__ __forceinline__ bool step(Ctx& c, uint32_t row, float4 (&x)[4]) {
+    const uint32_t flags = op.flags;
+    const bool live = row < op.rows, centre = !(flags & (F_RMSNORM | F_L2NORM));
+    if (!(flags & F_SRC_F32)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = h4_to_f4(make_uint2(__float_as_uint(x[i].x), __float_as_uint(x[i].y)));
+    }
+    if (flags & F_RESID) {
+      const uint2* p = reinterpret_cast<const uint2*>(op.p[4]) + static_cast<size_t>(live ? row : 0u) * (op.ldr >> 2) + v0;
+      uint2 h[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) h[i] = __ldcg(p + 32 * i);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add4(x[i], h4_to_f4(h[i]));
+    }
     if ((flags & F_ZERO_SRC) && live) {
+      float4* p = reinterpret_cast<float4*>(op.p[1]) + static_cast<size_t>(row) * (op.lds >> 2) + v0;
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (on[i]) const_cast<float4*>(src)[vi[i]] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) p[32 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-  } else {
-    const uint2* src = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[1]) +
-                                                      static_cast<size_t>(safe_row) * op.lds);
+    float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) x[i] = h4_to_f4(__ldcg(src + vi[i]));
-  }
-  if (flags & F_RESID) {
-    const uint2* res = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[4]) +
-                                                      static_cast<size_t>(safe_row) * op.ldr);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) add4(x[i], h4_to_f4(__ldcg(res + vi[i])));
-  }
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (!on[i]) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    sum += x[i].x + x[i].y + x[i].z + x[i].w;
-  }
-  // Each warp reduces its quarter to (sum, sum of squared deviations from its own mean); the
-  // four pairs are combined after ONE meeting in shared memory:
-  //   M2 = sum_w [ M2_w + n_w (mean_w - mean)^2 ]       (pairwise variance combination)
-  // which is as accurate as the two-pass form and saves its second group barrier.
-  const float inv_n = 1.0f / static_cast<float>(cols);
-  const float n_w = static_cast<float>(cols >> 2), inv_nw = 1.0f / n_w;
-  sum = warp_sum(sum);
-  const float mean_w = rms ? 0.f : sum * inv_nw;
-  float sq = 0.f;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    if (on[i]) {
-      const float a = x[i].x - mean_w, b = x[i].y - mean_w, d = x[i].z - mean_w, e = x[i].w - mean_w;
-      sq += a * a + b * b + d * d + e * e;
+    for (int i = 0; i < 4; ++i) {
+      if (lane + 32u * i >= per) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      sum += (x[i].x + x[i].y) + (x[i].z + x[i].w);
     }
-  sq = warp_sum(sq);
-  if (lane == 0) {
-    c.ctrl->ln_part[0][r_in][part] = sum;
-    c.ctrl->ln_part[1][r_in][part] = sq;
-  }
-  if (!group_sync(c, 0x431)) return false;
-  const float* p0 = c.ctrl->ln_part[0][r_in];
-  const float* p1 = c.ctrl->ln_part[1][r_in];
-  const float mean = rms ? 0.f : (p0[0] + p0[1] + p0[2] + p0[3]) * inv_n;
-  float m2 = p1[0] + p1[1] + p1[2] + p1[3];
-  if (!rms) {
+    const float n_w = static_cast<float>(per * 4u), inv_nw = 1.0f / n_w, inv_n = 1.0f / static_cast<float>(op.cols);
+    if (centre) sum = warp_sum(sum);
+    const float mean_w = centre ? sum * inv_nw : 0.f;
+    float sq = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float dm = p0[w] * inv_nw - mean;
-      m2 = fmaf(n_w * dm, dm, m2);
-    }
-  }
-  const float rstd = rsqrtf(m2 * inv_n + op.eps);
-  if (live) {
-    uint2* out = op.p[0] ? reinterpret_cast<uint2*>(reinterpret_cast<__half*>(op.p[0]) +
-                                                    static_cast<size_t>(row) * op.ldo)
-                         : nullptr;
-    float4* out2 = two ? reinterpret_cast<float4*>(reinterpret_cast<float*>(op.q[2]) +
-                                                   static_cast<size_t>(row) * cols)
-                       : nullptr;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (!on[i]) continue;
-      const float4 g = h4_to_f4(gv[i]);
-      const float4 b = rms ? make_float4(0.f, 0.f, 0.f, 0.f) : h4_to_f4(bv[i]);
-      float4 y;
-      y.x = (x[i].x - mean) * rstd * g.x + b.x;
-      y.y = (x[i].y - mean) * rstd * g.y + b.y;
-      y.z = (x[i].z - mean) * rstd * g.z + b.z;
-      y.w = (x[i].w - mean) * rstd * g.w + b.w;
-      if (out != nullptr) {
-        uint2 o;
-        o.x = pack_h2(y.x, y.y);
-        o.y = pack_h2(y.z, y.w);
-        out[vi[i]] = o;
+    for (int i = 0; i < 4; ++i)
+      if (lane + 32u * i < per) {
+        const float a = x[i].x - mean_w, b = x[i].y - mean_w, d = x[i].z - mean_w, e = x[i].w - mean_w;
+        sq += (a * a + b * b) + (d * d + e * e);
       }
-      if (out2 != nullptr) {
-        if (add_b2) add4(y, h4_to_f4(b2v[i]));
-        out2[vi[i]] = y;
+    sq = warp_sum(sq);
+    float mean = mean_w, m2 = sq;
+    if (group > 1u) {
+      const float2* meet = c.ctrl->ln_part[done & 1u] + (widx - part);
+      if (lane == 0) c.ctrl->ln_part[done & 1u][widx] = make_float2(sum, sq);
+      if (!group_sync(c, 0x431)) return false;
+      const float2 w0 = meet[0], w1 = meet[1];
+      float2 w2 = make_float2(0.f, 0.f), w3 = w2;
+      if (group == 4u) { w2 = meet[2]; w3 = meet[3]; }
+      m2 = (w0.y + w1.y) + (w2.y + w3.y);
+      if (centre) {
+        mean = ((w0.x + w1.x) + (w2.x + w3.x)) * inv_n;
+        const float d0 = w0.x * inv_nw - mean, d1 = w1.x * inv_nw - mean;
+        m2 = fmaf(n_w * d0, d0, fmaf(n_w * d1, d1, m2));
+        if (group == 4u) {
+          const float d2 = w2.x * inv_nw - mean, d3 = w3.x * inv_nw - mean;
+          m2 = fmaf(n_w * d2, d2, fmaf(n_w * d3, d3, m2));
+        }
       }
     }
+    ++done;
+    const float rstd = (flags & F_L2NORM) ? rsqrtf(m2) : rsqrtf(m2 * inv_n + op.eps);
+    if (!live) return true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 g = unpack(gv[i]), b = unpack(bv[i]);
+      x[i].x = (x[i].x - mean) * rstd * g.x + b.x;
+      x[i].y = (x[i].y - mean) * rstd * g.y + b.y;
+      x[i].z = (x[i].z - mean) * rstd * g.z + b.z;
+      x[i].w = (x[i].w - mean) * rstd * g.w + b.w;
+    }
+    if (op.p[0] != 0) {
+      uint2* o = reinterpret_cast<uint2*>(op.p[0]) + static_cast<size_t>(row) * (op.ldo >> 2) + v0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) o[32 * i] = make_uint2(pack_h2(x[i].x, x[i].y), pack_h2(x[i].z, x[i].w));
+    }
+    if (op.q[2] != 0) {
+      float4* o = reinterpret_cast<float4*>(op.q[2]) + static_cast<size_t>(row) * (op.cols >> 2) + v0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add4(x[i], unpack(b2v[i]));  // zero when there is no bias to pre-load
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (lane + 32u * i < per) o[32 * i] = x[i];
+    }
+    return true;
   }
-  return true;
+};
+__device__ __forceinline__ uint32_t layernorm_rows(Ctx& c, const OpDesc& op, uint32_t local, uint32_t widx,
+                                                   uint32_t lane) {
+  const uint32_t group = op.row_warps, per = op.cols / (4u * group), part = widx & (group - 1u);
+  NormRows n{op, lane, part, per, part * per + lane, widx, group, 0u, {}, {}, {}};
+  // a warp's k-th row: its item's rows in `parts` steps, then the CTA's next item
+  const uint32_t item_rows = (op.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
+  const uint32_t shift = (op.flags & F_ROW_SPLIT) ? 0u : group >> 1;  // log2 of the steps an item takes
+  const uint32_t items = (op.n_items - local + gridDim.x - 1u) / gridDim.x;  // this CTA's, this one included
+  const uint32_t steps = items << shift, first = local * item_rows + widx / group, per_step = kSimtWarps / group;
+  auto row_of = [&](uint32_t k) {
+    return first + (k >> shift) * gridDim.x * item_rows + (k & ((1u << shift) - 1u)) * per_step;
+  };
+  float4 x0[4], x1[4];
+  n.load(row_of(0), x0);
+  if (steps > 1u) n.load(row_of(1), x1);
+  n.constants();
+#pragma unroll 1
+  for (uint32_t k = 0;; k += 2u) {
+    if (!n.step(c, row_of(k), x0)) return 0u;
+    if (k + 2u < steps) n.load(row_of(k + 2u), x0);
+    if (k + 1u >= steps) break;
+    if (!n.step(c, row_of(k + 1u), x1)) return 0u;
+    if (k + 3u < steps) n.load(row_of(k + 3u), x1);
+    if (k + 2u >= steps) break;
+  }
+  return items;
 }
 
 // Arg-max item: one f16 row per 256-thread group. Each thread scans every 256th 16-byte
@@ -1700,7 +1758,7 @@ __device__ __noinline__ bool rowwise_split_item(Ctx& c, const OpDesc& op, uint32
 // partial results are merged by (larger value, then smaller index): the first index of the
 // row maximum, which is what XLA's (value, index) reduce returns
 // (reduction functors: mononn_engine/codegen/reduction_functor_generator.cc:296-441).
-__device__ __noinline__ bool argmax_item(Ctx& c, const OpDesc& op, uint32_t row, uint32_t widx,
+__device__ __forceinline__ bool argmax_item(Ctx& c, const OpDesc& op, uint32_t row, uint32_t widx,
                                          uint32_t lane, uint32_t tid_in_group) {
   const uint32_t nvec = op.cols >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(op.p[1]) +
@@ -1753,7 +1811,7 @@ __device__ __noinline__ bool argmax_item(Ctx& c, const OpDesc& op, uint32_t row,
 
 // Pooling at the largest token id: out[b, :] = src[b * seq + argmax(ids[b, :]), :], the first
 // maximum on ties (the end-of-text row of a CLIP text tower). One warp per output row.
-__device__ __noinline__ void rowsel_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
+__device__ __forceinline__ void rowsel_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
                                          uint32_t lane) {
   const uint32_t b = local * kRowsPerItem + warp_in_group;
   if (b >= op.rows) return;
@@ -1779,7 +1837,7 @@ __device__ __noinline__ void rowsel_item(const OpDesc& op, uint32_t local, uint3
 
 // out[i, j] = alpha * <a[i, :], b[j, :]> for two small f16 activations (the image-text logits
 // of a dual encoder: a few dozen rows each). One warp per row i, lanes over j.
-__device__ __noinline__ void pairdot_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
+__device__ __forceinline__ void pairdot_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
                                           uint32_t lane) {
   const uint32_t i = local * kRowsPerItem + warp_in_group;
   if (i >= op.M) return;
@@ -1814,7 +1872,7 @@ __device__ __noinline__ void pairdot_item(const OpDesc& op, uint32_t local, uint
 // that operand the convolution is a plain GEMM against the [out_channels, ky*kx*c] filter. The
 // reference runs these through CUTLASS implicit-GEMM fprop
 // (mononn_engine/core/op_impl/conv_impl.cc:36-106, 252-345).
-__device__ __noinline__ void patchify_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
+__device__ __forceinline__ void patchify_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
                                            uint32_t lane) {
   const uint32_t row = local * kRowsPerItem + warp_in_group;
   if (row >= op.rows) return;
@@ -1857,7 +1915,7 @@ __device__ __noinline__ void patchify_item(const OpDesc& op, uint32_t local, uin
 // `half` = 0, 1 of the row's TMEM quarter): each takes one 64-key half of every 128-key score
 // chunk (which is also one of the chunk's two P tiles) and 32 of the 64 output columns; the row
 // maximum and the row sum are combined through shared memory.
-__device__ __noinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_t local,
+__device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_t local,
                                             uint32_t tmem_base, uint32_t& a_cnt, uint32_t& acc_cnt,
                                             uint32_t quarter, uint32_t half, uint32_t lane,
                                             uint32_t tid_in_group) {
@@ -1912,10 +1970,16 @@ __device__ __noinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_t l
     uint8_t* tileV = c.a_ring_ptr + (cV % kASlots) * kSlotBytes + (row >> 6) * 8192u;
     // one 32-column load is in flight while the previous one is converted and stored
     auto convert = [&](const uint32_t (&r)[32], uint32_t c0) {
-      float v[32], bb[32];
-      lds32(bs + c0, bb);
+      float v[32];
+      const float4* bq = reinterpret_cast<const float4*>(bs + c0);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) + bb[i];
+      for (int i = 0; i < 8; ++i) {
+        const float4 b4 = bq[i];
+        v[4 * i] = __uint_as_float(r[4 * i]) + b4.x;
+        v[4 * i + 1] = __uint_as_float(r[4 * i + 1]) + b4.y;
+        v[4 * i + 2] = __uint_as_float(r[4 * i + 2]) + b4.z;
+        v[4 * i + 3] = __uint_as_float(r[4 * i + 3]) + b4.w;
+      }
       if (c0 < 128u) {
         uint8_t* tile = c.a_ring_ptr + (((c0 < 64u) ? cQ : cK) % kASlots) * kSlotBytes;
         const uint32_t chunk = (c0 & 63u) >> 3;
@@ -1938,13 +2002,13 @@ __device__ __noinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_t l
     uint32_t ra[32], rb[32];
     const uint32_t h32 = half * 32u;
     tc_ld32_issue(tQ + h32, ra);
-    tc_wait_ld();
+    tc_wait_ld(ra);
     tc_ld32_issue(tQ + 64u + h32, rb);
     convert(ra, h32);
-    tc_wait_ld();
+    tc_wait_ld(rb);
     tc_ld32_issue(tQ + 128u + h32, ra);
     convert(rb, 64u + h32);
-    tc_wait_ld();
+    tc_wait_ld(ra);
     convert(ra, 128u + h32);
     if (tid_in_group == 0) trace(*c.P, c.stage, TR_MARK0 + 5);
     // Every warp makes its part of the tiles visible to the tensor core (proxy fence) and counts
@@ -1979,14 +2043,28 @@ __device__ __noinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_t l
     // One key chunk, no causal mask, no position bias (the encoder case): the 64 scaled and masked
     // scores of this thread stay in registers between the maximum and the exponentials, so the
     // accumulator and the mask row are read once.
+    // (both loads in flight at once, then scaled in place: no second set of registers)
     float z[64];
+    {
+      uint32_t ra[32], rb[32];
+      tc_ld32_issue(tS + h64, ra);
+      tc_ld32_issue(tS + h64 + 32u, rb);
+      tc_wait_ld(ra);
+      tc_wait_ld(rb);
 #pragma unroll
-    for (uint32_t c0 = 0; c0 < 64u; c0 += 32u) {
-      float v[32], mk[32];
-      lds32(mb + h64 + c0, mk);
-      tc_ld32(tS + h64 + c0, v);
+      for (int i = 0; i < 32; ++i) {
+        z[i] = __uint_as_float(ra[i]);
+        z[32 + i] = __uint_as_float(rb[i]);
+      }
+    }
+    const float4* mq = reinterpret_cast<const float4*>(mb + h64);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) z[c0 + i] = fmaf(v[i], alpha, mk[i]);
+    for (int i = 0; i < 16; ++i) {
+      const float4 m = mq[i];
+      z[4 * i] = fmaf(z[4 * i], alpha, m.x);
+      z[4 * i + 1] = fmaf(z[4 * i + 1], alpha, m.y);
+      z[4 * i + 2] = fmaf(z[4 * i + 2], alpha, m.z);
+      z[4 * i + 3] = fmaf(z[4 * i + 3], alpha, m.w);
     }
     float m0 = z[0], m1 = z[1], m2 = z[2], m3 = z[3];
 #pragma unroll
@@ -2171,7 +2249,7 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
   uint32_t a_cnt = 0, acc_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
-    const StageDesc st = load_stage(P, s);
+    const StageDesc& st = load_stage(P, c.ctrl, 3u + widx, s, lane);
     uint4* slot = c.ctrl->desc[3 + widx];
     Item first{nullptr, 0};
     if (blockIdx.x < st.n_items) {
@@ -2240,8 +2318,10 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
             prefetch_row_consts(op, lane);
             WAIT_OR_RETURN(flag_wait_warp(c, op.flag, op.flag_target, 0x430));
           }
-          if (op.flags & F_ROW_SPLIT) {
-            WAIT_OR_RETURN(rowwise_split_item(c, op, it.local, widx, lane));
+          if (op.row_warps != 0u) {
+            const uint32_t n = layernorm_rows(c, op, it.local, widx, lane);
+            WAIT_OR_RETURN(n != 0u);
+            item += (n - 1u) * gridDim.x;
           } else {
             rowwise_item(op, it.local, widx, lane, P, s);
           }

@@ -53,7 +53,8 @@ struct TuningSpec {
   // warps count themselves in shared memory), 2 one per epilogue warp (each releases its own
   // stores), 1 one per CTA after a CTA-wide sync (always the case inside a cluster launch)
   uint32_t barrier_arrive = 0;
-  // 0 / 2: a LayerNorm with few rows shares each row among four warps; 1: always one warp per row
+  // 0 / 2: a LayerNorm with few rows shares each row among four warps; 1: never (as few as
+  // hold a row: one up to 512 columns, two up to 1024, four beyond)
   uint32_t row_split = 0;
   // 2: the GEMM that reads an attention's output shares its stage and waits on its arrival counter;
   // 3: only behind an attention that computes its own projections; 1: it keeps a stage of its own;

@@ -199,10 +199,14 @@ int validate_plan(const Plan& P, std::string* err) {
       case OP_EMBED:
       case OP_ASSEMBLE:
         if (d.cols == 0 || d.cols % 4 || d.cols > 2048) return bad(n + "row length");
-        if (d.flags & F_ROW_SPLIT) {
-          if (d.kind != OP_LAYERNORM || d.cols % 16 || d.cols > 1024 || (d.flags & (F_L2NORM | F_NO_NORM)))
-            return bad(n + "row split geometry");
-          if (d.n_items != (d.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem) return bad(n + "item count");
+        if (d.row_warps) {
+          if (d.kind != OP_LAYERNORM || (d.row_warps != 1 && d.row_warps != 2 && d.row_warps != 4) ||
+              d.cols % (4 * d.row_warps) || d.cols > d.row_warps * 512u || d.lds % 4 || d.ldo % 4 || d.ldr % 4 ||
+              (d.flags & F_NO_NORM))
+            return bad(n + "warps per row");
+          if ((d.flags & F_ROW_SPLIT) && d.row_warps != 4) return bad(n + "warps per row");
+          const uint32_t per_item = (d.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
+          if (d.n_items != (d.rows + per_item - 1) / per_item) return bad(n + "item count");
         } else if (d.n_items != (d.rows + kRowsPerItem - 1) / kRowsPerItem) return bad(n + "item count");
         if (op.p[0].space == SPACE_NONE && op.q[2].space == SPACE_NONE) return bad(n + "no output buffer");
         if (op.p[6].space == SPACE_NONE && d.kind != OP_LAYERNORM) return bad(n + "no scale pointer");
@@ -958,15 +962,26 @@ int schedule(const FGraph& g, const TuningSpec& spec_in, uint32_t sm_count, Plan
             if (err) *err = "layernorm " + o.name + ": row length must be <= 2048 and a multiple of 4";
             return MONONN_ERR_UNSUPPORTED;
           }
-          d.n_items = (o.rows + kRowsPerItem - 1) / kRowsPerItem;
-          // Few rows (batch 1): one warp per row leaves most CTAs idle while each row's load ->
-          // reduce -> normalise -> store chain runs on a single warp. Four warps per row, two rows
-          // per item, when all items still fit one wave of the CTAs.
-          if (spec_in.row_split != 1 && !(o.flags & (F_L2NORM | F_NO_NORM)) && o.cols % 16 == 0 && o.cols <= 1024 &&
-              (o.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem <= P.grid) {
-            d.flags |= F_ROW_SPLIT;
-            d.n_items = (o.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem;
+          // Warps per row. Few rows (batch 1): with one warp per row most CTAs are idle while each row's
+          // load -> reduce -> normalise -> store chain runs on a single warp, so four warps share a row
+          // when all items still fit one wave of the CTAs (BERT-base b1: 4 us of an inference). Many
+          // rows: as few as the 512 columns that a warp holds allow.
+          d.row_warps = 0;
+          if (!(o.flags & F_NO_NORM)) {
+            if (spec_in.row_split != 1 && o.cols % 16 == 0 && o.cols <= 2048 &&
+                (o.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem <= P.grid) {
+              d.row_warps = 4;
+              d.flags |= F_ROW_SPLIT;
+            } else if (o.cols <= 512) {
+              d.row_warps = 1;
+            } else if (o.cols <= 1024 && o.cols % 8 == 0) {
+              d.row_warps = 2;
+            } else if (o.cols % 16 == 0) {
+              d.row_warps = 4;
+            }
           }
+          const uint32_t rows_per_item = (d.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
+          d.n_items = (o.rows + rows_per_item - 1) / rows_per_item;
           po.p[0] = where[o.out];
           d.ldo = g.tensors[o.out].ld;
           po.p[1] = where[o.src];

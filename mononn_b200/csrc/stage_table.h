@@ -55,7 +55,7 @@ enum OpFlags : uint32_t {
   F_FUSED_QKV = 1u << 11,  // attention: the item first computes its own Q, K, V = x W_h + b_h
   F_POS_BIAS = 1u << 12,   // attention: additive f16 bias per (head, query, key), q[0] = [heads, seq, seq]
   F_RMSNORM = 1u << 13,    // row op: x * rsqrt(mean(x^2) + eps) * scale (no mean subtraction, no shift)
-  F_ROW_SPLIT = 1u << 14,  // LayerNorm: a row is shared by four warps (two rows per work item), for few rows
+  F_ROW_SPLIT = 1u << 14,  // LayerNorm of few rows: four warps to a row, two rows per work item
 };
 
 // Pointer slots p[0..7]; meaning per kind:
@@ -101,7 +101,8 @@ struct alignas(16) OpDesc {
   uint32_t rows;            // row count for row-wise ops
   uint32_t lds;             // leading dim of row-wise source
   uint32_t vocab;           // embed: word-table rows (ids are not clamped, as in the reference)
-  uint32_t pad0;
+  uint32_t row_warps;       // LayerNorm: warps that share a row (1, 2 or 4; at most 512 columns each),
+                            // 0: one warp per row (a row length that 4 x warps does not divide)
   uint32_t flag_target;     // row op that follows its producer GEMM inside one stage: arrivals to wait for
   uint32_t wait_target;     // GEMM that follows the attention it reads inside one stage: arrivals to wait for
   uint64_t p[8];
@@ -161,7 +162,7 @@ constexpr uint32_t kSimtThreads = 256;        // warps 4..11: epilogue / row-wis
 constexpr uint32_t kSimtWarps = kSimtThreads / 32;
 constexpr uint32_t kThreads = kRoleThreads + kSimtThreads;
 constexpr uint32_t kRowsPerItem = kSimtWarps;  // row-wise operators: one row per SIMT warp per work item
-constexpr uint32_t kSplitRowsPerItem = 2;      // LayerNorm with F_ROW_SPLIT: four warps per row
+constexpr uint32_t kSplitRowsPerItem = 2;      // LayerNorm with F_ROW_SPLIT
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTraceEvents = 16;  // per (CTA, stage) slots of the optional event trace
 constexpr uint32_t kAccCols = 256;  // two accumulator buffers of 256 columns
