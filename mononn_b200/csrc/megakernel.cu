@@ -174,21 +174,6 @@ __device__ __forceinline__ bool elect_one_sync() {
       "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred)::"memory");
   return pred != 0u;
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  __syncwarp();
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 // Issue only: the registers are valid after tc_wait_ld on them. Lets the following load be in
 // flight while the previous one is processed.
 __device__ __forceinline__ void tc_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
@@ -217,6 +202,25 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[32]) {
                :
                : "memory");
 }
+__device__ __forceinline__ void tc_ld_issue(uint32_t taddr, uint32_t (&r)[32]) { tc_ld32_issue(taddr, r); }
+__device__ __forceinline__ void tc_ld_issue(uint32_t taddr, uint32_t (&r)[16]) {
+  __syncwarp();
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                 "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+                 "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+                 "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]),
+                 "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   __syncwarp();
@@ -234,14 +238,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-// Polling uses relaxed loads: an acquire load in a spin loop would invalidate the SM's L1 on
-// every iteration, under the feet of the warps that are doing the stage's work. One acquire
-// load after the poll succeeds gives the ordering.
-__device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 // Thread-block cluster helpers: rank of this CTA, the shared::cluster address of a peer's copy of
 // a shared-memory object, a remote mbarrier arrival with release at cluster scope, the matching
@@ -280,9 +276,6 @@ __device__ __forceinline__ uint32_t ld_acquire_cta_smem(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
   return v;
-}
-__device__ __forceinline__ void fence_acq_rel_gpu() {
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t atom_add_acq_rel_cta_smem(uint32_t* p, uint32_t v) {
   uint32_t old;
@@ -327,6 +320,7 @@ struct Ctrl {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t group_bar;  // the eight epilogue warps (one arrival per warp and phase)
+  unsigned long long failure;  // notes of the wait that gave up first: stage, status code, wait site
   uint64_t cl_bar;     // first CTA of a cluster: one arrival per CTA of the cluster per stage
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -367,23 +361,50 @@ struct Ctx {
   uint8_t* store_stage;  // kStoreStageBytes after the control block: 2 KB per epilogue warp
   uint32_t stage;   // current stage (for status)
   uint32_t group_phase;  // parity of the next group_bar phase (epilogue warps only)
-  uint64_t timeout_ns;
 };
 
-__device__ __noinline__ void report_failure(const KernelParams* P, Ctrl* ctrl, uint32_t stage,
-                                            uint32_t code, uint32_t where) {
-  volatile uint32_t* af = &ctrl->abort_flag;
+// Every wait of this kernel is bounded. The code that gives up is inlined at each wait (a call would put
+// the whole kernel under the calling convention: state in memory around it, and no register beyond
+// the launch's share for any role), so it only takes notes in shared memory; the notes reach the
+// status word when the role returns (publish_failure).
+__device__ __forceinline__ uint32_t coarse_time() {
+  return static_cast<uint32_t>(globaltimer_ns() >> 10);  // units of 1.024 us
+}
+__device__ __forceinline__ bool give_up(const Ctx& c, uint32_t& t0, StatusCode code, uint32_t where, bool ask_others) {
+  volatile uint32_t* af = &c.ctrl->abort_flag;
+  if (*af) return true;
+  if (ask_others && *reinterpret_cast<volatile uint32_t*>(&c.P->status->code) != 0u) {
+    *af = 1;
+    return true;
+  }
+  const uint32_t now = coarse_time();
+  if (t0 == 0u) t0 = now | 1u;  // the timer is slow and most waits end before it is read
+  if (static_cast<int32_t>(now - t0 - c.P->timeout_us) <= 0) return false;
+  atomicCAS(&c.ctrl->failure, 0ull,
+            static_cast<unsigned long long>(c.stage) << 32 | static_cast<uint32_t>(code) << 16 | where);
   *af = 1;
-  KernelStatus* st = P->status;
-  if (atomicCAS(&st->code, 0u, code) == 0u) {
-    st->stage = stage;
-    st->cta = blockIdx.x;
-    st->where = where;
-    __threadfence();
-    if (P->host_flag != nullptr) {
-      *reinterpret_cast<volatile uint32_t*>(P->host_flag) = code;
-      __threadfence_system();
-    }
+  return true;
+}
+template <typename Test>
+__device__ __forceinline__ bool bounded_wait(const Ctx& c, StatusCode code, uint32_t where, bool ask_others, Test test) {
+  uint32_t t0 = 0;
+#pragma unroll 1
+  for (uint32_t it = 1; !test(); ++it)
+    if ((it & 63u) == 0u && give_up(c, t0, code, where, ask_others)) return false;
+  return true;
+}
+// One lane of each warp, on the abort path.
+__device__ __forceinline__ void publish_failure(const KernelParams& P, Ctrl* ctrl) {
+  const unsigned long long f = atomicExch(&ctrl->failure, 0ull);
+  const uint32_t code = (static_cast<uint32_t>(f) >> 16) & 0xffffu;
+  if (code == 0u || atomicCAS(&P.status->code, 0u, code) != 0u) return;
+  P.status->stage = static_cast<uint32_t>(f >> 32);
+  P.status->cta = blockIdx.x;
+  P.status->where = static_cast<uint32_t>(f) & 0xffffu;
+  __threadfence();
+  if (P.host_flag != nullptr) {
+    *reinterpret_cast<volatile uint32_t*>(P.host_flag) = code;
+    __threadfence_system();
   }
 }
 
@@ -404,31 +425,12 @@ __device__ __forceinline__ void trace(const KernelParams& P, uint32_t stage, uin
     P.trace[(static_cast<size_t>(blockIdx.x) * (P.stage_end - P.stage_begin) +
              (stage - P.stage_begin)) * kTraceEvents + ev] = globaltimer_ns();
 }
-// Bounded wait on an mbarrier phase. Returns false when the kernel is aborting. The slow
-// path is out of line so that the many wait sites stay a few instructions each.
-__device__ __noinline__ bool mbar_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t b,
-                                            uint32_t parity, uint32_t stage, uint32_t where) {
-  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
-  const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
-  uint32_t it = 0;
-  for (;;) {
-    if (mbar_try_wait(b, parity)) return true;
-    if ((++it & 63u) == 0u) {
-      if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > limit) {
-        report_failure(P, ctrl, stage, ST_MBARRIER_TIMEOUT, where);
-        return false;
-      }
-    }
-  }
+// Bounded wait on an mbarrier phase. Returns false when the kernel is aborting.
+__device__ __forceinline__ bool mbar_wait_at(const Ctx& c, uint32_t bar, uint32_t parity, uint32_t where) {
+  return bounded_wait(c, ST_MBARRIER_TIMEOUT, where, false, [=]() { return mbar_try_wait(bar, parity) != 0u; });
 }
-__device__ __forceinline__ bool mbar_wait(const Ctx& c, uint64_t* bar, uint32_t parity,
-                                          uint32_t where) {
-  const uint32_t b = smem_u32(bar);
-  if (mbar_try_wait(b, parity)) return true;
-  return mbar_wait_slow(c.P, c.ctrl, b, parity, c.stage, where);
+__device__ __forceinline__ bool mbar_wait(const Ctx& c, uint64_t* bar, uint32_t parity, uint32_t where) {
+  return mbar_wait_at(c, smem_u32(bar), parity, where);
 }
 
 // The counters are polled with acquire loads: the load that sees the count observes the last
@@ -437,108 +439,36 @@ __device__ __forceinline__ bool mbar_wait(const Ctx& c, uint64_t* bar, uint32_t 
 // acquire load at the end +7 us (one more L2 round trip per wait), a fence.acq_rel.gpu after a
 // relaxed poll +39 us (it also waits for this thread's own outstanding stores). A pause between
 // polls (__nanosleep) only delays the detection (+2 us at 32 ns).
-#ifndef MONONN_POLL_ACQUIRE
-#define MONONN_POLL_ACQUIRE 1  // 0: relaxed polls, then one acquire load
-#endif
 __device__ __forceinline__ uint32_t poll_load(const uint32_t* p) {
-#if MONONN_POLL_ACQUIRE
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-#else
-  return ld_relaxed_gpu(p);
-#endif
 }
-__device__ __forceinline__ void acquire_after_poll(const uint32_t* p) {
-#if MONONN_POLL_ACQUIRE
-  (void)p;
-#else
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  (void)v;
-#endif
-}
-#ifndef MONONN_ALL_POLL
-#define MONONN_ALL_POLL 0  // 1: every epilogue warp polls the global counter itself
-#endif
-#ifndef MONONN_POLL_SLEEP
-#define MONONN_POLL_SLEEP 0
-#endif
 // Bounded wait until every CTA has arrived for all stages before `stage`. Two threads per CTA
 // poll the global counter: the activation producer (its first tile load is the critical path of
 // a GEMM stage; routing it through a second hop measured 20 us slower over a whole inference)
 // and the first epilogue warp's lane 0, which then publishes the number of barriers seen in
 // shared memory for the other seven epilogue warps: some 300 pollers on the counter's L2 line
 // instead of 1300.
-__device__ __noinline__ bool grid_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t target,
-                                            uint32_t stage, uint32_t where) {
-  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
-  const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
-  uint32_t it = 0;
-  for (;;) {
-    if (static_cast<int32_t>(poll_load(P->barrier) - target) >= 0) {
-      acquire_after_poll(P->barrier);
-      return true;
-    }
-#if MONONN_POLL_SLEEP > 0
-    __nanosleep(MONONN_POLL_SLEEP);
-#endif
-    if ((++it & 31u) == 0u) {
-      if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      if (*reinterpret_cast<volatile uint32_t*>(&P->status->code) != 0u) {
-        *reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag) = 1;
-        return false;
-      }
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > limit) {
-        report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
-        return false;
-      }
-    }
-  }
-}
-// A global poller; with `announce` it also makes the shared-memory announcement.
+// With `announce` a global poller also makes the shared-memory announcement.
 __device__ __forceinline__ bool grid_wait(const Ctx& c, uint32_t stage, uint32_t where, bool announce) {
   const KernelParams& P = *c.P;
   if (stage == P.stage_begin) return true;
   const uint32_t target =
       P.epoch_base + (stage - P.stage_begin) * (gridDim.x / P.cluster) * (P.warp_arrive == 1u ? kSimtWarps : 1u);
-  bool ok = true;
-  if (static_cast<int32_t>(poll_load(P.barrier) - target) >= 0) {
-    acquire_after_poll(P.barrier);
-  } else {
-    ok = grid_wait_slow(c.P, c.ctrl, target, stage, where);
-  }
+  const bool ok = bounded_wait(c, ST_GRID_BARRIER_TIMEOUT, where, true,
+                               [&]() { return static_cast<int32_t>(poll_load(P.barrier) - target) >= 0; });
   if (ok && announce) st_release_cta_smem(&c.ctrl->barriers_seen, stage - P.stage_begin);
   return ok;
 }
 // Everybody else in the CTA: wait for the poller's announcement (acquire at CTA scope after the
 // poller's acquire at GPU scope orders the other CTAs' stores before this thread's loads).
-__device__ __noinline__ bool local_wait_slow(const KernelParams* P, Ctrl* ctrl, uint32_t need,
-                                             uint32_t stage, uint32_t where) {
-  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
-  const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
-  uint32_t it = 0;
-  for (;;) {
-    if (ld_acquire_cta_smem(&ctrl->barriers_seen) >= need) return true;
-    if ((++it & 63u) == 0u) {
-      if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > limit) {
-        report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
-        return false;
-      }
-    }
-  }
-}
 __device__ __forceinline__ bool grid_wait_local(const Ctx& c, uint32_t stage, uint32_t where) {
   const KernelParams& P = *c.P;
   if (stage == P.stage_begin) return true;
   const uint32_t need = stage - P.stage_begin;
-  if (ld_acquire_cta_smem(&c.ctrl->barriers_seen) >= need) return true;
-  return local_wait_slow(c.P, c.ctrl, need, stage, where);
+  return bounded_wait(c, ST_GRID_BARRIER_TIMEOUT, where, false,
+                      [&]() { return ld_acquire_cta_smem(&c.ctrl->barriers_seen) >= need; });
 }
 
 // Warp-collective variants for the epilogue warps: every lane gets the same answer, so a
@@ -551,11 +481,7 @@ __device__ __forceinline__ bool mbar_wait_warp(const Ctx& c, uint64_t* bar, uint
 __device__ __forceinline__ bool grid_wait_warp(const Ctx& c, uint32_t stage, uint32_t where) {
   bool ok = true;
   if ((threadIdx.x & 31u) == 0u)
-#if MONONN_ALL_POLL
-    ok = grid_wait(c, stage, where, threadIdx.x == kRoleThreads);
-#else
     ok = (threadIdx.x == kRoleThreads) ? grid_wait(c, stage, where, true) : grid_wait_local(c, stage, where);
-#endif
   return __all_sync(0xffffffffu, ok);
 }
 // A row op that shares a stage with the split-K GEMMs feeding it waits until all of their work
@@ -563,31 +489,6 @@ __device__ __forceinline__ bool grid_wait_warp(const Ctx& c, uint32_t stage, uin
 // with release).
 // Bounded like every wait; the waiting CTAs have no GEMM item left to do, so the GEMM items
 // never depend on a waiter.
-__device__ __noinline__ bool flag_wait_slow(const KernelParams* P, Ctrl* ctrl, const uint32_t* flag,
-                                            uint32_t target, uint32_t stage, uint32_t where) {
-  uint64_t t0 = 0;  // read at the first check below: the timer is slow and most waits end before it
-  const uint64_t limit = static_cast<uint64_t>(P->timeout_us) * 1000ull;
-  uint32_t it = 0;
-  for (;;) {
-    if (static_cast<int32_t>(poll_load(flag) - target) >= 0) {
-      acquire_after_poll(flag);
-      return true;
-    }
-    if ((++it & 31u) == 0u) {
-      if (*reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) return false;
-      if (*reinterpret_cast<volatile uint32_t*>(&P->status->code) != 0u) {
-        *reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag) = 1;
-        return false;
-      }
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > limit) {
-        report_failure(P, ctrl, stage, ST_GRID_BARRIER_TIMEOUT, where);
-        return false;
-      }
-    }
-  }
-}
 // The counter is never reset inside the kernel: like the grid-barrier counter it grows by the
 // same amount every launch, and the host passes the number of launches since it was last
 // cleared (flag_epoch), so the target is flag_epoch * arrivals-per-launch. No atomic with a
@@ -597,11 +498,8 @@ __device__ __forceinline__ bool flag_wait_warp(const Ctx& c, uint64_t counter, u
   if ((threadIdx.x & 31u) == 0u) {
     const uint32_t* flag = reinterpret_cast<const uint32_t*>(counter);
     const uint32_t target = c.P->flag_epoch * per_launch;
-    if (static_cast<int32_t>(poll_load(flag) - target) >= 0) {
-      acquire_after_poll(flag);
-    } else {
-      ok = flag_wait_slow(c.P, c.ctrl, flag, target, c.stage, where);
-    }
+    ok = bounded_wait(c, ST_GRID_BARRIER_TIMEOUT, where, true,
+                      [&]() { return static_cast<int32_t>(poll_load(flag) - target) >= 0; });
   }
   return __all_sync(0xffffffffu, ok);
 }
@@ -962,12 +860,10 @@ struct MmaRing {
   __device__ __forceinline__ uint32_t a_peek() const { return mbar_test_wait(a_full0 + a_slot * 8u, a_par); }
   __device__ __forceinline__ uint32_t b_peek() const { return mbar_test_wait(b_full0 + b_slot * 8u, b_par); }
   __device__ __forceinline__ bool a_wait(const Ctx& c, uint32_t where) const {
-    const uint32_t bar = a_full0 + a_slot * 8u;
-    return mbar_try_wait(bar, a_par) || mbar_wait_slow(c.P, c.ctrl, bar, a_par, c.stage, where);
+    return mbar_wait_at(c, a_full0 + a_slot * 8u, a_par, where);
   }
   __device__ __forceinline__ bool b_wait(const Ctx& c, uint32_t where) const {
-    const uint32_t bar = b_full0 + b_slot * 8u;
-    return mbar_try_wait(bar, b_par) || mbar_wait_slow(c.P, c.ctrl, bar, b_par, c.stage, where);
+    return mbar_wait_at(c, b_full0 + b_slot * 8u, b_par, where);
   }
   __device__ __forceinline__ void a_next() {
     if (++a_slot == kASlots) { a_slot = 0; a_par ^= 1u; }
@@ -1116,35 +1012,80 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
 // is kept compact (chunk loops are not unrolled, slow paths are out of line): the whole
 // kernel has to stay resident in the instruction cache across a layer's stages.
 // ----------------------------------------------------------------------------
-__device__ __forceinline__ float gelu_erf_f(float x) {
-  // erf by the rational form 1 - (a1 t + .. + a5 t^5) exp(-z^2), t = 1/(1 + p z), whose
-  // absolute error (1.5e-7) is far below the f16 resolution of the stored result
-  const float z = fabsf(x) * 0.70710678118654752f;
-  const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-  float p = fmaf(t, 1.061405429f, -1.453152027f);
-  p = fmaf(t, p, 1.421413741f);
-  p = fmaf(t, p, -0.284496736f);
-  p = fmaf(t, p, 0.254829592f);
-  const float e = 1.0f - p * t * __expf(-z * z);
-  return 0.5f * x * (1.0f + copysignf(e, x));
+// Two f32 operations in one instruction (the packed forms of sm_100).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// gelu(x) = x Phi(x) = max(x, 0) - |x| Phi(-|x|), with Phi(-a) = 2^q(a): log2 Phi(-a) is so smooth that a
+// polynomial of degree 7 (least squares on [0, 6], reweighted towards equal absolute error of a Phi(-a))
+// leaves 2.4e-7 of absolute error in gelu, its tail falls off by itself (negative leading term), and
+// one exponential is the only special-function operation. The rational form of erf with a reciprocal
+// and an exponential that stood here before was off by 4.7e-7 and took about twice the instructions.
+// (q is evaluated at -a. Its coefficients are held in register pairs for a whole tile: left to itself
+// the compiler moves each into a pair again in front of every packed instruction.)
+struct GeluConst {
+  float c[8];
+  __device__ __forceinline__ GeluConst()
+      : c{-0.99998665f, 1.1512747f, -0.4585138f, 0.05381008f, 0.00838564f, 0.00088752585f, 5.477368e-05f, 1.4344369e-06f} {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) asm volatile("" : "+f"(c[i]));
+  }
+};
+__device__ __forceinline__ float2 gelu_erf2(float2 x, const GeluConst& k) {
+  const float2 a = make_float2(fmaxf(-fabsf(x.x), -16.f), fmaxf(-fabsf(x.y), -16.f));
+  float2 q = fma2(splat2(k.c[7]), a, splat2(k.c[6]));
+#pragma unroll
+  for (int i = 5; i >= 0; --i) q = fma2(q, a, splat2(k.c[i]));
+  const float2 e = make_float2(fast_exp2(q.x), fast_exp2(q.y));
+  return fma2(a, e, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
 }
 
-__device__ __forceinline__ void apply_act16(float (&v)[16], uint32_t act) {
+template <int W>
+__device__ __forceinline__ void apply_act(float (&v)[W], uint32_t act, const GeluConst& gelu) {
   if (act == ACT_GELU_ERF) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = gelu_erf_f(v[i]);
+    for (int i = 0; i < W; i += 2) {
+      const float2 y = gelu_erf2(make_float2(v[i], v[i + 1]), gelu);
+      v[i] = y.x;
+      v[i + 1] = y.y;
+    }
   } else if (act == ACT_RELU) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
+    for (int i = 0; i < W; ++i) v[i] = fmaxf(v[i], 0.0f);
   } else if (act == ACT_QUICK_GELU) {
+    // x / (1 + exp(-1.702 x))
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __fdividef(v[i], 1.0f + __expf(-1.702f * v[i]));
+    for (int i = 0; i < W; ++i) v[i] *= fast_rcp(1.0f + fast_exp2(-2.4554669595930157f * v[i]));
   } else if (act == ACT_GELU_TANH) {
+    // 0.5 (1 + tanh u) = 1 / (1 + exp(-2u)), u = sqrt(2/pi) (x + 0.044715 x^3)
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < W; ++i) {
       const float u = 0.7978845608028654f * fmaf(0.044715f * v[i] * v[i], v[i], v[i]);
-      // 0.5 (1 + tanh u) = 1 / (1 + exp(-2u))
-      v[i] = __fdividef(v[i], 1.0f + __expf(-2.0f * u));
+      v[i] *= fast_rcp(1.0f + fast_exp2(-2.8853900817779268f * u));
     }
   }
 }
@@ -1177,11 +1118,6 @@ __device__ __forceinline__ void add_bias32(const __half* p, float (&mk)[32]) {
     }
   }
 }
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -1196,108 +1132,134 @@ __device__ __forceinline__ void add4(float4& a, const float4 b) {
 }
 
 // Accumulator row `quarter * 32 + lane` (TMEM lane = row) is shared by the two warps of the
-// quarter: warp `half` takes every other column group of the tile (groups of 32 columns, of 16
-// for tiles up to 32 wide so that both warps have work).
-__device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t, uint32_t tmem_acc,
-                                           uint32_t quarter, uint32_t half, uint32_t lane,
-                                           const float* bias_s, uint8_t* stg) {
-  const uint32_t grow = t.mt * 128u + quarter * 32u + lane;
-  const bool row_ok = grow < op.M;
+// quarter: warp `half` takes every other group of W columns of the tile (32; 16 for tiles up to 32
+// wide, so that both warps have work).
+//
+// Bound by the instructions its eight warps issue, two to a scheduler: 5.3 us for a 128 x 256 tile and
+// 8.8 us with GELU when it took 16 columns at a time with every choice inside the loop. A group is
+// one TMEM load now, issued while the group before it is worked on; additions and GELU's polynomial
+// are packed two to an instruction; row addresses are worked out once per tile.
+// Row-major results leave through the warp's staging block (32 rows x 64 bytes, swizzled), so that
+// four lanes write a row's 64 bytes: f32 reductions straight from the accumulator rows, 16 bytes in
+// each of 32 rows per instruction, were what the split-K tiles waited for.
+template <int W>
+__device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t, uint32_t tmem_acc, uint32_t quarter,
+                                              uint32_t half, uint32_t lane, const float* bias_s, uint8_t* stg) {
+  const uint32_t row0 = t.mt * 128u + quarter * 32u, n0 = t.nt * op.n_tile;
   const bool lead = (t.ks == 0);
-  const uint32_t n0 = t.nt * op.n_tile;
-  const uint32_t flags = op.flags, act = op.act, out_mode = op.out_mode, N = op.N;
-  const uint32_t ldo = op.ldo, ldr = op.ldr, n_tile = op.n_tile;
-  const float alpha = op.alpha;
-  const uint64_t pout = op.p[0], presid = op.p[2];
+  const uint32_t flags = op.flags, act = op.act, out_mode = op.out_mode, M = op.M, ldo = op.ldo;
+  const uint32_t n_cols = (op.N - n0 < op.n_tile) ? op.N - n0 : op.n_tile;  // a multiple of 16
   const bool bias_on = (flags & F_BIAS) && lead, resid_on = (flags & F_RESID) && lead;
-  // row-major f16 output: a 32-column group is collected in the warp's staging block (32 rows x
-  // 64 bytes, swizzled) and stored four lanes to a row instead of one row per lane
-  const bool staged = (out_mode == OUT_F16);
-  // transposed output: batch and row inside the batch of this thread's row, once per item
-  const uint32_t t_batch = (out_mode == OUT_F16_T) ? grow / op.rows_per_batch : 0u;
-  const uint32_t t_row = (out_mode == OUT_F16_T) ? grow - t_batch * op.rows_per_batch : 0u;
-  const uint32_t sw = (lane >> 1) & 3u;
-  const uint32_t gstep = (n_tile <= 32u) ? 16u : 32u;
+  const float alpha = op.alpha;
+  const uint32_t tmem = tmem_acc + ((quarter * 32u) << 16);
+  // this lane's places in the staging block: as the owner of a row, and as one of four lanes of row
+  // l4 + 8 j that move its 16-byte piece `piece`
+  const uint32_t sw = (lane >> 1) & 3u, l4 = lane >> 2, piece = lane & 3u;
+  uint8_t* const mine = stg + lane * 64u;
+  const uint8_t* const theirs = stg + l4 * 64u + ((piece ^ ((l4 >> 1) & 3u)) << 4);
+  const uint32_t esize = (out_mode == OUT_F16) ? 2u : 4u;
+  uint8_t* const out = reinterpret_cast<uint8_t*>(op.p[0]) + (static_cast<size_t>(row0 + l4) * ldo + n0) * esize + piece * 16u;
+  const size_t row_step = static_cast<size_t>(ldo) * 8u * esize;
+  const uint32_t rows_left = (row0 + l4 < M) ? M - row0 - l4 : 0u;  // row l4 + 8 j exists while 8 j < rows_left
+
+  const GeluConst gelu;
+  uint32_t r[W];
+  if (half * W < n_cols) tc_ld_issue(tmem + half * W, r);
 #pragma unroll 1
-  for (uint32_t g0 = half * gstep; g0 < n_tile; g0 += 2u * gstep) {
-    const uint32_t gw = (n_tile - g0 < gstep) ? n_tile - g0 : gstep;  // 16 or 32 columns
-#pragma unroll 1
-    for (uint32_t c0 = g0; c0 < g0 + gw; c0 += 16) {
-      float v[16];
-      tc_ld16(tmem_acc + ((quarter * 32u) << 16) + c0, v);
-      const uint32_t col = n0 + c0;
-      if (row_ok && col < N) {
-        if (alpha != 1.0f) {
+  for (uint32_t g0 = half * W; g0 < n_cols; g0 += 2u * W) {
+    float v[W];
+    tc_wait_ld(r);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] *= alpha;
-        }
-        if (bias_on) {
-          const float4* bq = reinterpret_cast<const float4*>(bias_s + c0);
+    for (int i = 0; i < W; ++i) v[i] = __uint_as_float(r[i]);
+    const bool more = g0 + 2u * W < n_cols;
+    const uint32_t width = (n_cols - g0 < W) ? n_cols - g0 : W;  // 16 or 32 columns
+    if (alpha != 1.0f) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 t = bq[i];
-            v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
-          }
-        }
-        apply_act16(v, act);
-        if (resid_on) {
-          if (flags & F_RESID_F32) {
-            const float4* r = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(presid) +
-                                                              static_cast<size_t>(grow) * ldr + col);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 x = __ldcg(r + i);
-              v[4 * i] += x.x; v[4 * i + 1] += x.y; v[4 * i + 2] += x.z; v[4 * i + 3] += x.w;
-            }
-          } else {
-            const uint2* r = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(presid) +
-                                                            static_cast<size_t>(grow) * ldr + col);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 x = h4_to_f4(__ldcg(r + i));
-              v[4 * i] += x.x; v[4 * i + 1] += x.y; v[4 * i + 2] += x.z; v[4 * i + 3] += x.w;
-            }
-          }
-        }
-        if (out_mode == OUT_F16) {
-          const uint32_t ch = (c0 - g0) >> 3;  // 0 or 2
-          *reinterpret_cast<uint4*>(stg + lane * 64u + ((ch ^ sw) << 4)) =
-              make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
-          *reinterpret_cast<uint4*>(stg + lane * 64u + (((ch + 1u) ^ sw) << 4)) =
-              make_uint4(pack_h2(v[8], v[9]), pack_h2(v[10], v[11]), pack_h2(v[12], v[13]), pack_h2(v[14], v[15]));
-        } else if (out_mode == OUT_F32_RED) {
-          float* o = reinterpret_cast<float*>(pout) + static_cast<size_t>(grow) * ldo + col;
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            red_add_f32x4(o + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else if (out_mode == OUT_F16_T) {
-          const uint32_t b = t_batch, rib = t_row;
-          const uint32_t ldt = op.ldt;
-          __half* o = reinterpret_cast<__half*>(pout) + (static_cast<size_t>(b) * N + col) * ldt + rib;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[static_cast<size_t>(i) * ldt] = __float2half_rn(v[i]);
-        } else {
-          float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(pout) +
-                                                static_cast<size_t>(grow) * ldo + col);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        }
-      }  // row_ok && col < N
+      for (int i = 0; i < W; ++i) v[i] *= alpha;
     }
-    if (staged) {
+    if (bias_on) {
+      const float4* bq = reinterpret_cast<const float4*>(bias_s + g0);
+#pragma unroll
+      for (int i = 0; i < W / 4; ++i) {
+        const float4 b = bq[i];
+        const float2 lo = add2(make_float2(v[4 * i], v[4 * i + 1]), make_float2(b.x, b.y));
+        const float2 hi = add2(make_float2(v[4 * i + 2], v[4 * i + 3]), make_float2(b.z, b.w));
+        v[4 * i] = lo.x; v[4 * i + 1] = lo.y; v[4 * i + 2] = hi.x; v[4 * i + 3] = hi.y;
+      }
+    }
+    apply_act<W>(v, act, gelu);
+    if (resid_on && row0 + lane < M) {
+      const size_t at = static_cast<size_t>(row0 + lane) * op.ldr + n0 + g0;
+      if (flags & F_RESID_F32) {
+        const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(op.p[2]) + at);
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i)
+          if (4u * i < width) {
+            const float4 x = __ldcg(q + i);
+            v[4 * i] += x.x; v[4 * i + 1] += x.y; v[4 * i + 2] += x.z; v[4 * i + 3] += x.w;
+          }
+      } else {
+        const uint2* q = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[2]) + at);
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i)
+          if (4u * i < width) {
+            const float4 x = h4_to_f4(__ldcg(q + i));
+            v[4 * i] += x.x; v[4 * i + 1] += x.y; v[4 * i + 2] += x.z; v[4 * i + 3] += x.w;
+          }
+      }
+    }
+    // (the next group's load goes out when this one's values have left its registers: before the stores)
+    if (out_mode == OUT_F16) {
+      uint32_t h[W / 2];
+#pragma unroll
+      for (int i = 0; i < W / 2; ++i) h[i] = pack_h2(v[2 * i], v[2 * i + 1]);
+      if (more) tc_ld_issue(tmem + g0 + 2u * W, r);
+#pragma unroll
+      for (uint32_t q = 0; q < W / 8; ++q)
+        *reinterpret_cast<uint4*>(mine + ((q ^ sw) << 4)) = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
       __syncwarp();
-      const uint32_t chunks = gw >> 3;  // 16-byte chunks per row in this group (2 or 4)
-      const uint32_t chunk_shift = chunks >> 1;  // log2(chunks): no division in the store loop
-      const uint32_t row0 = t.mt * 128u + quarter * 32u;
-      for (uint32_t idx = lane; idx < 32u * chunks; idx += 32u) {
-        const uint32_t r = idx >> chunk_shift, q = idx & (chunks - 1u);
-        const uint32_t gcol = n0 + g0 + q * 8u;
-        if (row0 + r < op.M && gcol < N)
-          *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(pout) + static_cast<size_t>(row0 + r) * ldo + gcol) =
-              *reinterpret_cast<const uint4*>(stg + r * 64u + ((q ^ ((r >> 1) & 3u)) << 4));
+      uint8_t* o = out + g0 * 2u;
+      if (piece * 8u < width) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          const uint4 x = *reinterpret_cast<const uint4*>(theirs + j * 512u);
+          if (8u * j < rows_left) *reinterpret_cast<uint4*>(o + j * row_step) = x;
+        }
       }
       __syncwarp();
+    } else if (out_mode == OUT_F16_T) {
+      const uint32_t grow = row0 + lane;
+      if (grow < M) {
+        const uint32_t b = grow / op.rows_per_batch, rib = grow - b * op.rows_per_batch, ldt = op.ldt;
+        __half* o = reinterpret_cast<__half*>(op.p[0]) + (static_cast<size_t>(b) * op.N + n0 + g0) * ldt + rib;
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          if (i < static_cast<int>(width)) o[static_cast<size_t>(i) * ldt] = __float2half_rn(v[i]);
+      }
+      if (more) tc_ld_issue(tmem + g0 + 2u * W, r);
+    } else {  // f32: reductions (split K, accumulating streams) or plain stores, 16 columns at a time
+      const bool reduce = out_mode == OUT_F32_RED;
+#pragma unroll
+      for (uint32_t h = 0; h < W; h += 16) {
+        if (h >= width) break;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          *reinterpret_cast<float4*>(mine + ((q ^ sw) << 4)) =
+              make_float4(v[h + 4 * q], v[h + 4 * q + 1], v[h + 4 * q + 2], v[h + 4 * q + 3]);
+        if (more && h + 16u == W) tc_ld_issue(tmem + g0 + 2u * W, r);  // (more to come: this group is full)
+        __syncwarp();
+        uint8_t* o = out + (g0 + h) * 4u;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          const float4 x = *reinterpret_cast<const float4*>(theirs + j * 512u);
+          if (8u * j < rows_left) {
+            float* d = reinterpret_cast<float*>(o + j * row_step);
+            if (reduce) red_add_f32x4(d, x.x, x.y, x.z, x.w);
+            else *reinterpret_cast<float4*>(d) = x;
+          }
+        }
+        __syncwarp();
+      }
     }
   }
 }
@@ -2285,8 +2247,12 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
           WAIT_OR_RETURN(mbar_wait_warp(c, &c.ctrl->acc_full[buf], (acc_cnt >> 1) & 1u, 0x401));
           if (tid_in_group == 0) trace(P, s, TR_MARK0 + 1);
           tc_fence_after();
-          gemm_epilogue(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s,
-                        c.store_stage + widx * 2048u);
+          if (op.n_tile > 32u)
+            gemm_epilogue<32>(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s,
+                              c.store_stage + widx * 2048u);
+          else
+            gemm_epilogue<16>(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s,
+                              c.store_stage + widx * 2048u);
           tc_fence_before();
           // A row op of this stage may wait for this item. The warps count themselves per
           // accumulator buffer in shared memory before they free the buffer (so the counts of two
@@ -2379,20 +2345,8 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
         mbar_arrive_remote_release_cluster(mapa_smem(smem_u32(&c.ctrl->cl_bar), 0u));
         if (cluster_ctarank() == 0u) {
           const uint32_t bar = smem_u32(&c.ctrl->cl_bar), parity = (s - P.stage_begin) & 1u;
-          bool ok = mbar_try_wait_acquire_cluster(bar, parity) != 0u;
-          if (!ok) {
-            const uint64_t t0 = globaltimer_ns();
-            for (uint32_t it = 1; !ok; ++it) {
-              ok = mbar_try_wait_acquire_cluster(bar, parity) != 0u;
-              if (!ok && (it & 63u) == 0u) {
-                if (*reinterpret_cast<volatile uint32_t*>(&c.ctrl->abort_flag)) break;
-                if (globaltimer_ns() - t0 > c.timeout_ns) {
-                  report_failure(c.P, c.ctrl, s, ST_GRID_BARRIER_TIMEOUT, 0x440);
-                  break;
-                }
-              }
-            }
-          }
+          const bool ok = bounded_wait(c, ST_GRID_BARRIER_TIMEOUT, 0x440, true,
+                                       [=]() { return mbar_try_wait_acquire_cluster(bar, parity) != 0u; });
           if (ok) red_release_gpu_add(P.barrier, 1u);
         }
       } else {
@@ -2434,6 +2388,7 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
     mbar_init(smem_u32(&ctrl->group_bar), kSimtWarps);
     mbar_init(smem_u32(&ctrl->cl_bar), P.cluster);
     ctrl->abort_flag = 0;
+    ctrl->failure = 0;
     ctrl->barriers_seen = 0;
     ctrl->warps_done = 0;
     ctrl->items_done[0] = ctrl->items_done[1] = 0;
@@ -2475,17 +2430,20 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
   c.store_stage = base + kASlots * kSlotBytes + kBSlots * kBSlotBytes + kCtrlBytes;
   c.stage = P.stage_begin;
   c.group_phase = 0;
-  c.timeout_ns = static_cast<uint64_t>(P.timeout_us) * 1000ull;
 
-  // 384 threads share the 64 K registers: 168 each, which every role fits without spilling.
+  // The launch gives every thread 168 registers (384 x 168 = 64 512). The first four warps need 72; what
+  // they leave goes to the epilogue warps: 128 x 72 + 256 x 216 = 64 512.
   if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == 0) role_weight_producer(c, lane);
     else if (warp == 1) role_act_producer(c, lane);
     else if (warp == 2) role_mma(c, tmem_base, lane);
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     role_simt(c, tmem_base, threadIdx.x - kRoleThreads);
   }
   __syncwarp();
+  if (lane == 0u && *reinterpret_cast<volatile uint32_t*>(&ctrl->abort_flag)) publish_failure(P, ctrl);
 
   // Teardown. On the abort path give copies and MMAs still in flight time to land
   // before the shared memory and TMEM they target are released.
