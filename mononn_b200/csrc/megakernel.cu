@@ -202,25 +202,6 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[32]) {
                :
                : "memory");
 }
-__device__ __forceinline__ void tc_ld_issue(uint32_t taddr, uint32_t (&r)[32]) { tc_ld32_issue(taddr, r); }
-__device__ __forceinline__ void tc_ld_issue(uint32_t taddr, uint32_t (&r)[16]) {
-  __syncwarp();
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-               "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                 "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-                 "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                 "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]),
-                 "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-               :
-               : "memory");
-}
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   __syncwarp();
@@ -1132,8 +1113,9 @@ __device__ __forceinline__ void add4(float4& a, const float4 b) {
 }
 
 // Accumulator row `quarter * 32 + lane` (TMEM lane = row) is shared by the two warps of the
-// quarter: warp `half` takes every other group of W columns of the tile (32; 16 for tiles up to 32
-// wide, so that both warps have work).
+// quarter: warp `half` takes every other group of 32 columns of the tile. (Tiles up to 32 wide leave half
+// of the warps without work. The two warps of a quarter share a scheduler, so a second instance of
+// this code for groups of 16 bought them nothing, and its 24 KB cost more than it: see role_simt.)
 //
 // Bound by the instructions its eight warps issue, two to a scheduler: 5.3 us for a 128 x 256 tile and
 // 8.8 us with GELU when it took 16 columns at a time with every choice inside the loop. A group is
@@ -1142,7 +1124,6 @@ __device__ __forceinline__ void add4(float4& a, const float4 b) {
 // Row-major results leave through the warp's staging block (32 rows x 64 bytes, swizzled), so that
 // four lanes write a row's 64 bytes: f32 reductions straight from the accumulator rows, 16 bytes in
 // each of 32 rows per instruction, were what the split-K tiles waited for.
-template <int W>
 __device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t, uint32_t tmem_acc, uint32_t quarter,
                                               uint32_t half, uint32_t lane, const float* bias_s, uint8_t* stg) {
   const uint32_t row0 = t.mt * 128u + quarter * 32u, n0 = t.nt * op.n_tile;
@@ -1162,9 +1143,10 @@ __device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t
   const size_t row_step = static_cast<size_t>(ldo) * 8u * esize;
   const uint32_t rows_left = (row0 + l4 < M) ? M - row0 - l4 : 0u;  // row l4 + 8 j exists while 8 j < rows_left
 
+  constexpr int W = 32;
   const GeluConst gelu;
   uint32_t r[W];
-  if (half * W < n_cols) tc_ld_issue(tmem + half * W, r);
+  if (half * W < n_cols) tc_ld32_issue(tmem + half * W, r);
 #pragma unroll 1
   for (uint32_t g0 = half * W; g0 < n_cols; g0 += 2u * W) {
     float v[W];
@@ -1213,7 +1195,7 @@ __device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t
       uint32_t h[W / 2];
 #pragma unroll
       for (int i = 0; i < W / 2; ++i) h[i] = pack_h2(v[2 * i], v[2 * i + 1]);
-      if (more) tc_ld_issue(tmem + g0 + 2u * W, r);
+      if (more) tc_ld32_issue(tmem + g0 + 2u * W, r);
 #pragma unroll
       for (uint32_t q = 0; q < W / 8; ++q)
         *reinterpret_cast<uint4*>(mine + ((q ^ sw) << 4)) = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
@@ -1236,7 +1218,7 @@ __device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t
         for (int i = 0; i < W; ++i)
           if (i < static_cast<int>(width)) o[static_cast<size_t>(i) * ldt] = __float2half_rn(v[i]);
       }
-      if (more) tc_ld_issue(tmem + g0 + 2u * W, r);
+      if (more) tc_ld32_issue(tmem + g0 + 2u * W, r);
     } else {  // f32: reductions (split K, accumulating streams) or plain stores, 16 columns at a time
       const bool reduce = out_mode == OUT_F32_RED;
 #pragma unroll
@@ -1246,7 +1228,7 @@ __device__ __forceinline__ void gemm_epilogue(const OpDesc& op, const GemmTile t
         for (uint32_t q = 0; q < 4; ++q)
           *reinterpret_cast<float4*>(mine + ((q ^ sw) << 4)) =
               make_float4(v[h + 4 * q], v[h + 4 * q + 1], v[h + 4 * q + 2], v[h + 4 * q + 3]);
-        if (more && h + 16u == W) tc_ld_issue(tmem + g0 + 2u * W, r);  // (more to come: this group is full)
+        if (more && h + 16u == W) tc_ld32_issue(tmem + g0 + 2u * W, r);  // (more to come: this group is full)
         __syncwarp();
         uint8_t* o = out + (g0 + h) * 4u;
 #pragma unroll
@@ -1460,39 +1442,7 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
 #pragma unroll
       for (int i = 0; i < 8; ++i) bv[i] = make_uint2(0u, 0u);
     }
-    if (!no_norm && !l2 && out != nullptr) {
-      // the common LayerNorm: the per-item choices are made once here, not per 8-byte group (a
-      // branch costs a warp that is alone on its scheduler some twenty cycles)
-      const bool two = (out2 != nullptr);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t vi = i * 32u + lane;
-        if (vi < nvec) {
-          const float4 g = h4_to_f4(gv[i]), b = h4_to_f4(bv[i]);
-          float4 y;
-          y.x = (x[i].x - mean) * rstd * g.x + b.x;
-          y.y = (x[i].y - mean) * rstd * g.y + b.y;
-          y.z = (x[i].z - mean) * rstd * g.z + b.z;
-          y.w = (x[i].w - mean) * rstd * g.w + b.w;
-          uint2 o;
-          o.x = pack_h2(y.x, y.y);
-          o.y = pack_h2(y.z, y.w);
-          out[vi] = o;
-          x[i] = y;
-        }
-      }
-      if (two) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t vi = i * 32u + lane;
-          if (vi < nvec) {
-            float4 y = x[i];
-            add4(y, h4_to_f4(b2v[i]));  // zero when there is no bias to pre-load
-            out2[vi] = y;
-          }
-        }
-      }
-    } else {
+    {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const uint32_t vi = i * 32u + lane;
@@ -1549,7 +1499,8 @@ __device__ __forceinline__ void prefetch_row_consts(const OpDesc& op, uint32_t l
 // 3 us, and with one row per warp and nothing in flight behind it the rows of a large batch took
 // 4 us a wave (6144 rows of 1024: 25 us for 63 MB of L2 traffic), rows of 2048 columns, read three
 // times, four times that. So a warp has two rows in registers: it works on one while the loads of
-// the next are under way. Everything is inline and small enough not to spill: with the counters
+// the next are under way. (One instance of the row's code: a loop unrolled over two rows is 20 KB more,
+// BERT-base b8 +2.8 %, and with three or four rows in registers everything is 2.5 % slower.) Everything is inline and small enough not to spill: with the counters
 // polled by acquire loads, L1 holds nothing for long and a spilled register is an L2 round trip.
 //
 // The warps that share a row meet once in shared memory with (sum, sum of squared deviations from
@@ -1701,16 +1652,13 @@ __device__ __forceinline__ uint32_t layernorm_rows(Ctx& c, const OpDesc& op, uin
   };
   float4 x0[4], x1[4];
   n.load(row_of(0), x0);
-  if (steps > 1u) n.load(row_of(1), x1);
   n.constants();
 #pragma unroll 1
-  for (uint32_t k = 0;; k += 2u) {
+  for (uint32_t k = 0; k < steps; ++k) {
+    if (k + 1u < steps) n.load(row_of(k + 1u), x1);
     if (!n.step(c, row_of(k), x0)) return 0u;
-    if (k + 2u < steps) n.load(row_of(k + 2u), x0);
-    if (k + 1u >= steps) break;
-    if (!n.step(c, row_of(k + 1u), x1)) return 0u;
-    if (k + 3u < steps) n.load(row_of(k + 3u), x1);
-    if (k + 2u >= steps) break;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x0[i] = x1[i];
   }
   return items;
 }
@@ -1931,7 +1879,7 @@ __device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_
     const uint32_t tQ = tmem_base + kAttnQkvCol + ((quarter * 32u) << 16);
     uint8_t* tileV = c.a_ring_ptr + (cV % kASlots) * kSlotBytes + (row >> 6) * 8192u;
     // one 32-column load is in flight while the previous one is converted and stored
-    auto convert = [&](const uint32_t (&r)[32], uint32_t c0) {
+    auto convert = [&](const uint32_t (&r)[32], uint32_t c0, bool values) {
       float v[32];
       const float4* bq = reinterpret_cast<const float4*>(bs + c0);
 #pragma unroll
@@ -1942,7 +1890,7 @@ __device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_
         v[4 * i + 2] = __uint_as_float(r[4 * i + 2]) + b4.z;
         v[4 * i + 3] = __uint_as_float(r[4 * i + 3]) + b4.w;
       }
-      if (c0 < 128u) {
+      if (!values) {
         uint8_t* tile = c.a_ring_ptr + (((c0 < 64u) ? cQ : cK) % kASlots) * kSlotBytes;
         const uint32_t chunk = (c0 & 63u) >> 3;
 #pragma unroll
@@ -1966,12 +1914,12 @@ __device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_
     tc_ld32_issue(tQ + h32, ra);
     tc_wait_ld(ra);
     tc_ld32_issue(tQ + 64u + h32, rb);
-    convert(ra, h32);
+    convert(ra, h32, false);
     tc_wait_ld(rb);
     tc_ld32_issue(tQ + 128u + h32, ra);
-    convert(rb, 64u + h32);
+    convert(rb, 64u + h32, false);
     tc_wait_ld(ra);
-    convert(ra, 128u + h32);
+    convert(ra, 128u + h32, true);
     if (tid_in_group == 0) trace(*c.P, c.stage, TR_MARK0 + 5);
     // Every warp makes its part of the tiles visible to the tensor core (proxy fence) and counts
     // itself; the warp that counts last hands the three tiles to the MMA issuer. Nobody waits
@@ -2203,6 +2151,11 @@ __device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_
 
 // ----------------------------------------------------------------------------
 // Role: epilogue + SIMT stages + grid barrier (warps 4..11)
+//
+// The whole kernel is some 210 KB of instructions, of which a layer runs about half, and the instruction
+// cache is what a stage's first pass through each part pays for: code that nothing in a graph runs
+// still costs it (24 KB of it made BERT-base b1 3 % slower, 41 KB 5.5 %, all sizes alike). So each
+// kind of work has one instance of its code here, also where a second one would take fewer instructions.
 // ----------------------------------------------------------------------------
 __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
   const KernelParams& P = *c.P;
@@ -2247,12 +2200,7 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
           WAIT_OR_RETURN(mbar_wait_warp(c, &c.ctrl->acc_full[buf], (acc_cnt >> 1) & 1u, 0x401));
           if (tid_in_group == 0) trace(P, s, TR_MARK0 + 1);
           tc_fence_after();
-          if (op.n_tile > 32u)
-            gemm_epilogue<32>(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s,
-                              c.store_stage + widx * 2048u);
-          else
-            gemm_epilogue<16>(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s,
-                              c.store_stage + widx * 2048u);
+          gemm_epilogue(op, tile, tmem_base + buf * kAccCols, quarter, half, lane, bias_s, c.store_stage + widx * 2048u);
           tc_fence_before();
           // A row op of this stage may wait for this item. The warps count themselves per
           // accumulator buffer in shared memory before they free the buffer (so the counts of two
