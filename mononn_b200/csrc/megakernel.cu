@@ -1801,23 +1801,33 @@ __device__ __forceinline__ void patchify_item(const OpDesc& op, uint32_t local, 
   const uint32_t per_row = C * kw;
   const uint32_t step_ky = 32u / per_row, step_kx = (32u % per_row) / C, step_c = 32u % C;
   uint32_t ky = lane / per_row, kx = (lane % per_row) / C, ch = lane % C;
-#pragma unroll 4
-  for (uint32_t j = lane; j < op.cols; j += 32u) {
-    const uint32_t y = y0 + ky, x = x0 + kx;  // a wrapped (negative) coordinate fails the bound test
-    float v = 0.f;
-    if (j < valid && y < Himg && x < Wimg) v = src[((static_cast<size_t>(b) * C + ch) * Himg + y) * Wimg + x];
-    dst[j] = __float2half_rn(v);
-    ch += step_c;
-    if (ch >= C) {
-      ch -= C;
-      ++kx;
+  // Bound by the latency of the pixel reads: none of them can move above the store of the element before
+  // it, so eight are issued before the first store.
+  constexpr uint32_t kBatch = 8;
+  const float* const img = src + static_cast<size_t>(b) * C * Himg * Wimg;
+#pragma unroll 1
+  for (uint32_t j0 = lane; j0 < op.cols; j0 += 32u * kBatch) {
+    float v[kBatch];
+#pragma unroll
+    for (uint32_t i = 0; i < kBatch; ++i) {
+      const uint32_t y = y0 + ky, x = x0 + kx;  // a wrapped (negative) coordinate fails the bound test
+      v[i] = 0.f;
+      if (j0 + 32u * i < valid && y < Himg && x < Wimg) v[i] = img[(static_cast<size_t>(ch) * Himg + y) * Wimg + x];
+      ch += step_c;
+      if (ch >= C) {
+        ch -= C;
+        ++kx;
+      }
+      kx += step_kx;
+      if (kx >= kw) {
+        kx -= kw;
+        ++ky;
+      }
+      ky += step_ky;
     }
-    kx += step_kx;
-    if (kx >= kw) {
-      kx -= kw;
-      ++ky;
-    }
-    ky += step_ky;
+#pragma unroll
+    for (uint32_t i = 0; i < kBatch; ++i)
+      if (j0 + 32u * i < op.cols) dst[j0 + 32u * i] = __float2half_rn(v[i]);
   }
 }
 
