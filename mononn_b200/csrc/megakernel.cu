@@ -1010,6 +1010,14 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
@@ -1021,28 +1029,32 @@ __device__ __forceinline__ float fast_rcp(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// gelu(x) = x Phi(x) = max(x, 0) - |x| Phi(-|x|), with Phi(-a) = 2^q(a): log2 Phi(-a) is so smooth that a
-// polynomial of degree 7 (least squares on [0, 6], reweighted towards equal absolute error of a Phi(-a))
-// leaves 2.4e-7 of absolute error in gelu, its tail falls off by itself (negative leading term), and
-// one exponential is the only special-function operation. The rational form of erf with a reciprocal
-// and an exponential that stood here before was off by 4.7e-7 and took about twice the instructions.
-// (q is evaluated at -a. Its coefficients are held in register pairs for a whole tile: left to itself
-// the compiler moves each into a pair again in front of every packed instruction.)
-struct GeluConst {
-  float c[8];
+// gelu(x) = x/2 (1 + erf(x / sqrt 2)), erf by the rational form 1 - (a1 t + .. + a5 t^5) exp(-z^2) with
+// t = 1 / (1 + p z) (Abramowitz and Stegun 7.1.26, absolute error 1.5e-7), two values at a time. A NaN
+// comes out as one, and towards zero the result keeps 5e-7 of relative error.
+// (max(x, 0) - |x| 2^q(|x|), one exponential and no reciprocal, stood here for a while: its two maxima
+// turned a NaN into 0, and its relative error below 0.05 was 9e-6.)
+// The constants are held in registers for a whole tile: left to itself the compiler moves each into
+// a register pair again in front of every packed instruction.
+struct GeluConst {  // (the coefficients of erf / 2, which saves the multiplication at the end: exact)
+  float p, one, a1, a2, a3, a4, a5, nlog2e, half;
   __device__ __forceinline__ GeluConst()
-      : c{-0.99998665f, 1.1512747f, -0.4585138f, 0.05381008f, 0.00838564f, 0.00088752585f, 5.477368e-05f, 1.4344369e-06f} {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) asm volatile("" : "+f"(c[i]));
+      : p(0.3275911f), one(1.0f), a1(0.5f * -0.254829592f), a2(0.5f * 0.284496736f), a3(0.5f * -1.421413741f),
+        a4(0.5f * 1.453152027f), a5(0.5f * -1.061405429f), nlog2e(-1.4426950408889634f), half(0.5f) {
+    asm volatile("" : "+f"(p), "+f"(one), "+f"(a1), "+f"(a2), "+f"(a3), "+f"(a4), "+f"(a5), "+f"(nlog2e), "+f"(half));
   }
 };
 __device__ __forceinline__ float2 gelu_erf2(float2 x, const GeluConst& k) {
-  const float2 a = make_float2(fmaxf(-fabsf(x.x), -16.f), fmaxf(-fabsf(x.y), -16.f));
-  float2 q = fma2(splat2(k.c[7]), a, splat2(k.c[6]));
-#pragma unroll
-  for (int i = 5; i >= 0; --i) q = fma2(q, a, splat2(k.c[i]));
-  const float2 e = make_float2(fast_exp2(q.x), fast_exp2(q.y));
-  return fma2(a, e, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+  const float2 z = make_float2(fabsf(x.x) * 0.70710678118654752f, fabsf(x.y) * 0.70710678118654752f);
+  const float2 d = fma2(splat2(k.p), z, splat2(k.one));
+  const float2 t = make_float2(fast_rcp(d.x), fast_rcp(d.y));
+  float2 q = fma2(t, splat2(k.a5), splat2(k.a4));
+  q = fma2(t, q, splat2(k.a3));
+  q = fma2(t, q, splat2(k.a2));
+  q = fma2(t, q, splat2(k.a1));
+  const float2 w = mul2(mul2(z, z), splat2(k.nlog2e));
+  const float2 e = fma2(mul2(q, t), make_float2(fast_exp2(w.x), fast_exp2(w.y)), splat2(k.half));  // erf(|z|) / 2
+  return mul2(x, add2(splat2(k.half), make_float2(copysignf(e.x, x.x), copysignf(e.y, x.y))));
 }
 
 template <int W>
@@ -1060,13 +1072,13 @@ __device__ __forceinline__ void apply_act(float (&v)[W], uint32_t act, const Gel
   } else if (act == ACT_QUICK_GELU) {
     // x / (1 + exp(-1.702 x))
 #pragma unroll
-    for (int i = 0; i < W; ++i) v[i] *= fast_rcp(1.0f + fast_exp2(-2.4554669595930157f * v[i]));
+    for (int i = 0; i < W; ++i) v[i] *= fast_rcp(1.0f + fast_exp2(-1.702f * v[i] * 1.4426950408889634f));
   } else if (act == ACT_GELU_TANH) {
     // 0.5 (1 + tanh u) = 1 / (1 + exp(-2u)), u = sqrt(2/pi) (x + 0.044715 x^3)
 #pragma unroll
     for (int i = 0; i < W; ++i) {
       const float u = 0.7978845608028654f * fmaf(0.044715f * v[i] * v[i], v[i], v[i]);
-      v[i] *= fast_rcp(1.0f + fast_exp2(-2.8853900817779268f * u));
+      v[i] *= fast_rcp(1.0f + fast_exp2(-2.0f * u * 1.4426950408889634f));
     }
   }
 }
