@@ -1518,12 +1518,14 @@ __device__ __forceinline__ void prefetch_row_consts(const OpDesc& op, uint32_t l
 // The warps that share a row meet once in shared memory with (sum, sum of squared deviations from
 // their own mean), combined pairwise:
 //   M2 = sum_w [ M2_w + n_w (mean_w - mean)^2 ]
-// which is as accurate as the two-pass form. The meeting place is double buffered, so one barrier a
-// row is enough. Returns the number of work items done (local, local + gridDim.x, ..), 0 on abort.
+// which is as accurate as the two-pass form. There are two meeting places, used by turns: the one of the
+// group barrier's phase. Whoever writes to one again has passed the barrier after the one that its
+// readers waited for, so one barrier a row is enough, from one operator of a stage to the next too (a
+// count that begins anew with each operator let a fast warp write while a slow one read). Returns the number of work items done (local, local + gridDim.x, ..), 0 on abort.
 struct NormRows {
   const OpDesc& op;
   uint32_t lane, part, per, v0;  // this warp's part of a row: vectors v0 + 32 i, while lane + 32 i < per
-  uint32_t widx, group, done;    // group: warps per row
+  uint32_t widx, group;          // group: warps per row
   uint2 gv[4], bv[4], b2v[4];    // scale, shift and pre-load bias of those columns, for all rows
 
   __device__ __forceinline__ void constants() {
@@ -1605,8 +1607,9 @@ struct NormRows {
     sq = warp_sum(sq);
     float mean = mean_w, m2 = sq;
     if (group > 1u) {
-      const float2* meet = c.ctrl->ln_part[done & 1u] + (widx - part);
-      if (lane == 0) c.ctrl->ln_part[done & 1u][widx] = make_float2(sum, sq);
+      float2* const place = c.ctrl->ln_part[c.group_phase];
+      const float2* meet = place + (widx - part);
+      if (lane == 0) place[widx] = make_float2(sum, sq);
       if (!group_sync(c, 0x431)) return false;
       const float2 w0 = meet[0], w1 = meet[1];
       float2 w2 = make_float2(0.f, 0.f), w3 = w2;
@@ -1622,7 +1625,6 @@ struct NormRows {
         }
       }
     }
-    ++done;
     const float rstd = (flags & F_L2NORM) ? rsqrtf(m2) : rsqrtf(m2 * inv_n + op.eps);
     if (!live) return true;
 #pragma unroll
@@ -1653,7 +1655,7 @@ struct NormRows {
 __device__ __forceinline__ uint32_t layernorm_rows(Ctx& c, const OpDesc& op, uint32_t local, uint32_t widx,
                                                    uint32_t lane) {
   const uint32_t group = op.row_warps, per = op.cols / (4u * group), part = widx & (group - 1u);
-  NormRows n{op, lane, part, per, part * per + lane, widx, group, 0u, {}, {}, {}};
+  NormRows n{op, lane, part, per, part * per + lane, widx, group, {}, {}, {}};
   // a warp's k-th row: its item's rows in `parts` steps, then the CTA's next item
   const uint32_t item_rows = (op.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
   const uint32_t shift = (op.flags & F_ROW_SPLIT) ? 0u : group >> 1;  // log2 of the steps an item takes
