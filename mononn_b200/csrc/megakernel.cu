@@ -301,6 +301,7 @@ struct Ctrl {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t group_bar;  // the eight epilogue warps (one arrival per warp and phase)
+  uint64_t row_bar[6];  // warps that share a LayerNorm row: four pairs, two fours
   unsigned long long failure;  // notes of the wait that gave up first: stage, status code, wait site
   uint64_t cl_bar;     // first CTA of a cluster: one arrival per CTA of the cluster per stage
   uint32_t tmem_base;
@@ -316,7 +317,7 @@ struct Ctrl {
   float mask_row[384];      // additive key mask of the current attention tile (log2 units)
   float row_max[2][128];    // attention: row maximum / row sum over each warp half's columns,
   float row_sum[2][128];    // exchanged between the two threads that share a query row
-  float2 ln_part[2][kSimtWarps];  // LayerNorm rows shared by several warps: per-warp (sum, squared deviations)
+  alignas(16) float4 ln_part[2][kSimtWarps];  // LayerNorm rows shared by four warps: what each has (see NormRows)
   float red_val[kSimtWarps];  // arg-max: per-warp partial results of the current row
   uint32_t red_idx[kSimtWarps];
   // Shared-memory copies of the operator descriptor each role is working on: slot 0 weight
@@ -342,6 +343,7 @@ struct Ctx {
   uint8_t* store_stage;  // kStoreStageBytes after the control block: 2 KB per epilogue warp
   uint32_t stage;   // current stage (for status)
   uint32_t group_phase;  // parity of the next group_bar phase (epilogue warps only)
+  uint32_t row_phase;    // the same for this warp's row_bar: bit 0 as one of a pair, bit 1 as one of four
 };
 
 // Every wait of this kernel is bounded. The code that gives up is inlined at each wait (a call would put
@@ -491,14 +493,17 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar) {
 }
 // Barrier across the 256 epilogue threads built on an mbarrier so that, unlike bar.sync,
 // the wait is bounded when a warp has already left on the abort path.
-__device__ __forceinline__ bool group_sync(Ctx& c, uint32_t where) {
+__device__ __forceinline__ bool warps_meet(const Ctx& c, uint32_t bar, uint32_t parity, uint32_t where) {
   // one arrival per warp (the warp barrier orders the other lanes' accesses before it): 256
   // arrivals on one shared-memory word would serialise for a quarter of a microsecond
   __syncwarp();
-  if ((threadIdx.x & 31u) == 0u) mbar_arrive(smem_u32(&c.ctrl->group_bar));
-  const bool ok = mbar_wait(c, &c.ctrl->group_bar, c.group_phase, where);
+  if ((threadIdx.x & 31u) == 0u) mbar_arrive(bar);
+  return __all_sync(0xffffffffu, mbar_wait_at(c, bar, parity, where));
+}
+__device__ __forceinline__ bool group_sync(Ctx& c, uint32_t where) {
+  const bool ok = warps_meet(c, smem_u32(&c.ctrl->group_bar), c.group_phase, where);
   c.group_phase ^= 1u;
-  return __all_sync(0xffffffffu, ok);
+  return ok;
 }
 
 #define WAIT_OR_RETURN(expr) \
@@ -1264,35 +1269,21 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Sources of one row of a row-wise op (LayerNorm or embedding): up to three addends.
+// Sources of one embedding row: up to three addends.
 struct RowSrc {
-  const float4* f32;   // f32 accumulator row (LayerNorm), cleared after reading when `zero`
-  const uint2* h0;     // f16 row: LayerNorm source, or the gathered word row
-  const uint2* h1;     // f16 row: residual, or the position row
-  const uint2* h2;     // f16 row: token-type row
-  bool zero;
+  const uint2* h0;  // the gathered word row, or the patch / prefix row
+  const uint2* h1;  // position row
+  const uint2* h2;  // token-type row, or the patch bias
 };
-// Loads only: the optional clearing of the f32 source is a separate step, because a store
-// between the loads would keep the compiler from issuing them back to back.
 __device__ __forceinline__ float4 row_chunk(const RowSrc& s, uint32_t vi) {
-  float4 a;
-  if (s.f32 != nullptr) {
-    a = __ldcg(s.f32 + vi);
-  } else {
-    a = h4_to_f4(__ldcg(s.h0 + vi));
-  }
+  float4 a = h4_to_f4(__ldcg(s.h0 + vi));
   if (s.h1 != nullptr) add4(a, h4_to_f4(__ldcg(s.h1 + vi)));
   if (s.h2 != nullptr) add4(a, h4_to_f4(__ldcg(s.h2 + vi)));
   return a;
 }
-__device__ __forceinline__ void row_emit(float4 a, float mean, float rstd, uint32_t vi,
-                                         uint2 gv, uint2 bv, uint2 b2v, uint2* out, float4* out2,
-                                         bool add_bias2, bool no_norm, bool l2 = false) {
-  float4 g = h4_to_f4(gv), b = h4_to_f4(bv);
-  if (l2) {
-    g = make_float4(1.f, 1.f, 1.f, 1.f);
-    b = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+__device__ __forceinline__ void row_emit(float4 a, float mean, float rstd, uint32_t vi, uint2 gv, uint2 bv, uint2 b2v,
+                                         uint2* out, float4* out2, bool add_bias2, bool no_norm) {
+  const float4 g = h4_to_f4(gv), b = h4_to_f4(bv);
   float4 y = a;
   if (!no_norm) {
     y.x = (a.x - mean) * rstd * g.x + b.x;
@@ -1312,19 +1303,19 @@ __device__ __forceinline__ void row_emit(float4 a, float mean, float rstd, uint3
   }
 }
 
-// LayerNorm / embedding item: eight rows, one warp each. Rows up to 1024 columns stay in
-// registers between the statistics and the normalisation; wider rows are re-read.
-__device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group,
-                                          uint32_t lane, const KernelParams& P, uint32_t stage) {
+// Embedding item (looked-up or assembled rows, with a LayerNorm or without): eight rows, one warp each.
+// Rows up to 1024 columns stay in registers between the statistics and the normalisation; wider
+// rows are re-read. (The norms of the layers: NormRows below.)
+__device__ __forceinline__ void embed_item(const OpDesc& op, uint32_t local, uint32_t warp_in_group, uint32_t lane,
+                                           const KernelParams& P, uint32_t stage) {
   const uint32_t row = local * kRowsPerItem + warp_in_group;
   if (row >= op.rows) return;
   const bool mark = (warp_in_group == 0 && lane == 0);
   if (mark) trace(P, stage, TR_MARK0);
   const uint32_t cols = op.cols, nvec = cols >> 2, flags = op.flags;
-  const bool embed = (op.kind == OP_EMBED), assemble = (op.kind == OP_ASSEMBLE);
-  const bool no_norm = (flags & F_NO_NORM) != 0u, l2 = (flags & F_L2NORM) != 0u, rms = (flags & F_RMSNORM) != 0u;
-  RowSrc s{nullptr, nullptr, nullptr, nullptr, false};
-  if (assemble) {
+  const bool no_norm = (flags & F_NO_NORM) != 0u;
+  RowSrc s{nullptr, nullptr, nullptr};
+  if (op.kind == OP_ASSEMBLE) {
     // token row t of batch b: the first k_col rows come from a constant table (class token),
     // the others from the patch GEMM's output plus its bias; every row adds its position row
     const uint32_t t = row % op.seq, b = row / op.seq, prefix = op.k_col;
@@ -1339,7 +1330,7 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
     }
     s.h1 = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[4]) +
                                           static_cast<size_t>(t) * cols);
-  } else if (embed) {
+  } else {
     const int32_t id = reinterpret_cast<const int32_t*>(op.p[1])[row];
     s.h0 = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[3]) +
                                           static_cast<int64_t>(id) * cols);
@@ -1355,23 +1346,11 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
       const int32_t m = reinterpret_cast<const int32_t*>(op.q[0])[row];
       reinterpret_cast<float*>(op.q[1])[row] = (1.0f - static_cast<float>(m)) * op.alpha;
     }
-  } else {
-    if (flags & F_SRC_F32) {
-      s.f32 = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(op.p[1]) +
-                                              static_cast<size_t>(row) * op.lds);
-      s.zero = (flags & F_ZERO_SRC) != 0u;
-    } else {
-      s.h0 = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[1]) +
-                                            static_cast<size_t>(row) * op.lds);
-    }
-    if (flags & F_RESID)
-      s.h1 = reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(op.p[4]) +
-                                            static_cast<size_t>(row) * op.ldr);
   }
-  // (row ops without normalisation still get valid scale/shift pointers from the host, so
+  // (rows without normalisation still get valid scale/shift pointers from the host, so
   // that the loads below stay unconditional)
-  const uint2* gamma = reinterpret_cast<const uint2*>((embed || assemble) ? op.p[6] : op.p[2]);
-  const uint2* beta = reinterpret_cast<const uint2*>((embed || assemble) ? op.p[7] : op.p[3]);
+  const uint2* gamma = reinterpret_cast<const uint2*>(op.p[6]);
+  const uint2* beta = reinterpret_cast<const uint2*>(op.p[7]);
   uint2* out = op.p[0] ? reinterpret_cast<uint2*>(reinterpret_cast<__half*>(op.p[0]) +
                                                   static_cast<size_t>(row) * op.ldo)
                        : nullptr;
@@ -1384,18 +1363,15 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
   const bool add_bias2 = (out2 != nullptr) && (bias2 != nullptr);
   if (nvec <= 256u) {
     // Every global load of the row is issued before anything waits on one of them. The
-    // loops are straight-line code (source kind decided outside, out-of-range chunks read
-    // chunk 0 and are zeroed afterwards): a branch between two loads would make the
-    // hardware wait for the first before issuing the second.
+    // loops are straight-line code (out-of-range chunks read chunk 0 and are zeroed
+    // afterwards): a branch between two loads would make the hardware wait for the first
+    // before issuing the second.
     float4 x[8];
     uint2 gv[8], bv[8], b2v[8];
     uint32_t vj[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) vj[i] = (i * 32u + lane < nvec) ? i * 32u + lane : 0u;
-    if (s.f32 != nullptr) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = __ldcg(s.f32 + vj[i]);
-    } else {
+    {
       uint2 h[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) h[i] = __ldcg(s.h0 + vj[i]);
@@ -1428,12 +1404,6 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
 #pragma unroll
       for (int i = 0; i < 8; ++i) add4(x[i], h4_to_f4(h[i]));
     }
-    if (s.zero) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i * 32u + lane < nvec)
-          const_cast<float4*>(s.f32)[i * 32u + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -1441,7 +1411,7 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
       sum += x[i].x + x[i].y + x[i].z + x[i].w;
     }
     if (mark) trace(P, stage, TR_MARK0 + 1);
-    const float mean = (l2 || rms) ? 0.f : warp_sum(sum) * inv_n;
+    const float mean = warp_sum(sum) * inv_n;
     float sq = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -1449,17 +1419,11 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
         const float a = x[i].x - mean, b = x[i].y - mean, c = x[i].z - mean, d = x[i].w - mean;
         sq += a * a + b * b + c * c + d * d;
       }
-    const float rstd = l2 ? rsqrtf(warp_sum(sq)) : rsqrtf(warp_sum(sq) * inv_n + eps);
-    if (rms) {  // no shift: the host binds the scale vector as the shift pointer too
+    const float rstd = rsqrtf(warp_sum(sq) * inv_n + eps);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) bv[i] = make_uint2(0u, 0u);
-    }
-    {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t vi = i * 32u + lane;
-        if (vi < nvec) row_emit(x[i], mean, rstd, vi, gv[i], bv[i], b2v[i], out, out2, add_bias2, no_norm, l2);
-      }
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t vi = i * 32u + lane;
+      if (vi < nvec) row_emit(x[i], mean, rstd, vi, gv[i], bv[i], b2v[i], out, out2, add_bias2, no_norm);
     }
   } else {
     // wide rows: three passes over the (L2-resident) sources
@@ -1469,7 +1433,7 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
       const float4 a = row_chunk(s, vi);
       sum += a.x + a.y + a.z + a.w;
     }
-    const float mean = (l2 || rms) ? 0.f : warp_sum(sum) * inv_n;
+    const float mean = warp_sum(sum) * inv_n;
     float sq = 0.f;
 #pragma unroll 1
     for (uint32_t vi = lane; vi < nvec; vi += 32u) {
@@ -1477,22 +1441,19 @@ __device__ __forceinline__ void rowwise_item(const OpDesc& op, uint32_t local, u
       const float e = a.x - mean, f = a.y - mean, g = a.z - mean, h = a.w - mean;
       sq += e * e + f * f + g * g + h * h;
     }
-    const float rstd = l2 ? rsqrtf(warp_sum(sq)) : rsqrtf(warp_sum(sq) * inv_n + eps);
+    const float rstd = rsqrtf(warp_sum(sq) * inv_n + eps);
 #pragma unroll 1
-    for (uint32_t vi = lane; vi < nvec; vi += 32u) {
-      const float4 a = row_chunk(s, vi);
-      if (s.zero) const_cast<float4*>(s.f32)[vi] = make_float4(0.f, 0.f, 0.f, 0.f);
-      row_emit(a, mean, rstd, vi, __ldg(gamma + vi), rms ? make_uint2(0u, 0u) : __ldg(beta + vi),
-               add_bias2 ? __ldg(bias2 + vi) : make_uint2(0u, 0u), out, out2, add_bias2, no_norm, l2);
-    }
+    for (uint32_t vi = lane; vi < nvec; vi += 32u)
+      row_emit(row_chunk(s, vi), mean, rstd, vi, __ldg(gamma + vi), __ldg(beta + vi),
+               add_bias2 ? __ldg(bias2 + vi) : make_uint2(0u, 0u), out, out2, add_bias2, no_norm);
   }
   if (mark) trace(P, stage, TR_MARK0 + 2);
 }
 
 // Scale, shift and pre-load bias of a row op are small constants that every layer reads once.
 // The weight stream (larger than L2) evicts them between their uses, so a row op asks for them
-// again while it waits for its inputs (grid barrier or arrival counter): the loads in
-// rowwise_item then hit L2 instead of paying an HBM round trip on the critical path.
+// again while it waits for its inputs (grid barrier or arrival counter): its loads
+// then hit L2 instead of paying an HBM round trip on the critical path.
 __device__ __forceinline__ void prefetch_row_consts(const OpDesc& op, uint32_t lane) {
   const bool alt = (op.kind == OP_EMBED || op.kind == OP_ASSEMBLE);
   const uint64_t g = alt ? op.p[6] : op.p[2], b = alt ? op.p[7] : op.p[3], b2 = op.q[3];
@@ -1511,26 +1472,34 @@ __device__ __forceinline__ void prefetch_row_consts(const OpDesc& op, uint32_t l
 // 3 us, and with one row per warp and nothing in flight behind it the rows of a large batch took
 // 4 us a wave (6144 rows of 1024: 25 us for 63 MB of L2 traffic), rows of 2048 columns, read three
 // times, four times that. So a warp has two rows in registers: it works on one while the loads of
-// the next are under way. (One instance of the row's code: a loop unrolled over two rows is 20 KB more,
-// BERT-base b8 +2.8 %, and with three or four rows in registers everything is 2.5 % slower.) Everything is inline and small enough not to spill: with the counters
-// polled by acquire loads, L1 holds nothing for long and a spilled register is an L2 round trip.
+// the next are under way. (One instance of the row's code: a loop unrolled over two rows is 20 KB
+// more, BERT-base b8 +2.8 %, and with three or four rows in registers everything is 2.5 % slower.)
+// Everything is inline and small enough not to spill: with the counters polled by acquire loads, L1
+// holds nothing for long and a spilled register is an L2 round trip.
 //
-// The warps that share a row meet once in shared memory with (sum, sum of squared deviations from
-// their own mean), combined pairwise:
+// Two warps (rows of 513 to 1024 columns) add in the order of one: lane l of a single warp would add its
+// vectors l, l + 32, .. one after another, so the first warp has the first half of those rounds, each
+// shows the other its lanes' sums, and both go on as one would. Two meetings a row, and results that
+// do not depend on the split, bit for bit. (Both rows' vectors in one warp need no meeting, but 19 KB
+// of code and spills.)
+// Four warps (few rows, or rows beyond 1024 columns) meet once with (sum, sum of squared deviations from
+// their own mean, columns and their reciprocal), combined pairwise, which is as accurate as the two passes:
 //   M2 = sum_w [ M2_w + n_w (mean_w - mean)^2 ]
-// which is as accurate as the two-pass form. There are two meeting places, used by turns: the one of the
-// group barrier's phase. Whoever writes to one again has passed the barrier after the one that its
-// readers waited for, so one barrier a row is enough, from one operator of a stage to the next too (a
-// count that begins anew with each operator let a fast warp write while a slow one read). Returns the number of work items done (local, local + gridDim.x, ..), 0 on abort.
+// What a warp shows is written to one of two places by turns, from one operator to the next too: it was
+// read before the barrier in between, so nobody still reads what is overwritten.
+// Returns the number of work items done (local, local + gridDim.x, ..), 0 on abort.
 struct NormRows {
   const OpDesc& op;
   uint32_t lane, part, per, v0;  // this warp's part of a row: vectors v0 + 32 i, while lane + 32 i < per
   uint32_t widx, group;          // group: warps per row
+  float n_w, inv_w, inv_n;       // columns of this part, its reciprocal and the one of a whole row's
   uint2 gv[4], bv[4], b2v[4];    // scale, shift and pre-load bias of those columns, for all rows
 
   __device__ __forceinline__ void constants() {
     const bool plain = (op.flags & F_L2NORM) != 0u, centre = !(op.flags & (F_RMSNORM | F_L2NORM));
     const bool b2 = op.q[2] != 0 && op.q[3] != 0;
+    inv_n = 1.0f / static_cast<float>(op.cols);  // (here: while the first row's loads are under way)
+    inv_w = 1.0f / n_w;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       gv[i] = make_uint2(0x3c003c00u, 0x3c003c00u);  // 1, 1, 1, 1
@@ -1546,6 +1515,14 @@ struct NormRows {
   static __device__ __forceinline__ float4 unpack(uint2 h) {
     asm volatile("" : "+r"(h.x), "+r"(h.y));
     return h4_to_f4(h);
+  }
+
+  // The warps of a row meet at a barrier of their own, so that none waits for another row's loads.
+  __device__ __forceinline__ uint32_t row_phase(const Ctx& c) const { return (group == 2u ? c.row_phase : c.row_phase >> 1) & 1u; }
+  __device__ __forceinline__ bool meet(Ctx& c, uint32_t where) const {
+    const uint32_t bar = smem_u32(&c.ctrl->row_bar[group == 2u ? widx >> 1 : 4u + (widx >> 2)]), parity = row_phase(c);
+    c.row_phase ^= group >> 1;
+    return warps_meet(c, bar, parity, where);
   }
 
   __device__ __forceinline__ void load(uint32_t row, float4 (&x)[4]) const {
@@ -1565,6 +1542,16 @@ struct NormRows {
           x[i].y = __uint_as_float(h.y);
         }
     }
+  }
+  // A lane's sum over its vectors of the row, in the order in which one warp would add them.
+  __device__ __forceinline__ bool in_order(Ctx& c, const float (&p)[4], float& s) const {
+    float4* const box = reinterpret_cast<float4*>(c.store_stage + widx * 2048u + row_phase(c) * 512u) + lane;
+    *box = make_float4(p[0], p[1], p[2], p[3]);
+    if (!meet(c, 0x431)) return false;
+    // the first part's sums, then the second's
+    const float4 f = *(part ? box - 128 : box), l = *(part ? box : box + 128);
+    s = f.x + f.y + f.z + f.w + l.x + l.y + l.z + l.w;
+    return true;
   }
   __device__ __forceinline__ bool step(Ctx& c, uint32_t row, float4 (&x)[4]) {
     const uint32_t flags = op.flags;
@@ -1588,41 +1575,44 @@ struct NormRows {
       for (int i = 0; i < 4; ++i)
         if (lane + 32u * i < per) p[32 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (lane + 32u * i >= per) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      sum += (x[i].x + x[i].y) + (x[i].z + x[i].w);
-    }
-    const float n_w = static_cast<float>(per * 4u), inv_nw = 1.0f / n_w, inv_n = 1.0f / static_cast<float>(op.cols);
-    if (centre) sum = warp_sum(sum);
-    const float mean_w = centre ? sum * inv_nw : 0.f;
-    float sq = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      if (lane + 32u * i < per) {
-        const float a = x[i].x - mean_w, b = x[i].y - mean_w, d = x[i].z - mean_w, e = x[i].w - mean_w;
-        sq += (a * a + b * b) + (d * d + e * e);
+      if (lane + 32u * i >= per) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+
+    float p[4], sum = 0.f, mean = 0.f;
+    if (centre) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = x[i].x + x[i].y + x[i].z + x[i].w;
+      sum = p[0] + p[1] + p[2] + p[3];
+      if (__builtin_expect(group == 2u, 0)) {
+        if (!in_order(c, p, sum)) return false;
       }
-    sq = warp_sum(sq);
-    float mean = mean_w, m2 = sq;
-    if (group > 1u) {
-      float2* const place = c.ctrl->ln_part[c.group_phase];
-      const float2* meet = place + (widx - part);
-      if (lane == 0) place[widx] = make_float2(sum, sq);
-      if (!group_sync(c, 0x431)) return false;
-      const float2 w0 = meet[0], w1 = meet[1];
-      float2 w2 = make_float2(0.f, 0.f), w3 = w2;
-      if (group == 4u) { w2 = meet[2]; w3 = meet[3]; }
-      m2 = (w0.y + w1.y) + (w2.y + w3.y);
+      sum = warp_sum(sum);
+      mean = sum * (group == 4u ? inv_w : inv_n);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      p[i] = 0.f;
+      if (lane + 32u * i < per) {
+        const float a = x[i].x - mean, b = x[i].y - mean, d = x[i].z - mean, e = x[i].w - mean;
+        p[i] = a * a + b * b + d * d + e * e;
+      }
+    }
+    float m2 = p[0] + p[1] + p[2] + p[3];
+    if (__builtin_expect(group == 2u, 0)) {
+      if (!in_order(c, p, m2)) return false;
+    }
+    m2 = warp_sum(m2);
+    if (group == 4u) {
+      float4* const all = c.ctrl->ln_part[row_phase(c)] + (widx - part);
+      if (lane == 0) all[part] = make_float4(sum, m2, n_w, inv_w);
+      if (!meet(c, 0x431)) return false;
+      const float4 w0 = all[0], w1 = all[1], w2 = all[2], w3 = all[3];
+      m2 = w0.y + w1.y + w2.y + w3.y;
       if (centre) {
-        mean = ((w0.x + w1.x) + (w2.x + w3.x)) * inv_n;
-        const float d0 = w0.x * inv_nw - mean, d1 = w1.x * inv_nw - mean;
-        m2 = fmaf(n_w * d0, d0, fmaf(n_w * d1, d1, m2));
-        if (group == 4u) {
-          const float d2 = w2.x * inv_nw - mean, d3 = w3.x * inv_nw - mean;
-          m2 = fmaf(n_w * d2, d2, fmaf(n_w * d3, d3, m2));
-        }
+        mean = (w0.x + w1.x + w2.x + w3.x) * inv_n;
+        const float d0 = w0.x * w0.w - mean, d1 = w1.x * w1.w - mean, d2 = w2.x * w2.w - mean, d3 = w3.x * w3.w - mean;
+        m2 = fmaf(w3.z * d3, d3, fmaf(w2.z * d2, d2, fmaf(w1.z * d1, d1, fmaf(w0.z * d0, d0, m2))));
       }
     }
     const float rstd = (flags & F_L2NORM) ? rsqrtf(m2) : rsqrtf(m2 * inv_n + op.eps);
@@ -1654,9 +1644,12 @@ struct NormRows {
 };
 __device__ __forceinline__ uint32_t layernorm_rows(Ctx& c, const OpDesc& op, uint32_t local, uint32_t widx,
                                                    uint32_t lane) {
-  const uint32_t group = op.row_warps, per = op.cols / (4u * group), part = widx & (group - 1u);
-  NormRows n{op, lane, part, per, part * per + lane, widx, group, {}, {}, {}};
-  // a warp's k-th row: its item's rows in `parts` steps, then the CTA's next item
+  const uint32_t group = op.row_warps, part = widx & (group - 1u), nvec = op.cols >> 2;
+  // vectors of a part (two warps: in whole rounds of 32; the last part has what is left)
+  const uint32_t share = (group == 2u) ? (nvec + 63u) / 64u * 32u : (nvec + group - 1u) / group;
+  const uint32_t per = (part + 1u == group) ? nvec - part * share : share;
+  NormRows n{op, lane, part, per, part * share + lane, widx, group, static_cast<float>(per * 4u), 0.f, 0.f, {}, {}, {}};
+  // a warp's k-th row: its item's rows in 2^shift steps, then the CTA's next item
   const uint32_t item_rows = (op.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
   const uint32_t shift = (op.flags & F_ROW_SPLIT) ? 0u : group >> 1;  // log2 of the steps an item takes
   const uint32_t items = (op.n_items - local + gridDim.x - 1u) / gridDim.x;  // this CTA's, this one included
@@ -1674,6 +1667,8 @@ __device__ __forceinline__ uint32_t layernorm_rows(Ctx& c, const OpDesc& op, uin
 #pragma unroll
     for (int i = 0; i < 4; ++i) x0[i] = x1[i];
   }
+  // the staging blocks are the warps' own again in the next item
+  if (group == 2u && !n.meet(c, 0x432)) return 0u;
   return items;
 }
 
@@ -2256,12 +2251,12 @@ __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
             prefetch_row_consts(op, lane);
             WAIT_OR_RETURN(flag_wait_warp(c, op.flag, op.flag_target, 0x430));
           }
-          if (op.row_warps != 0u) {
+          if (op.kind == OP_LAYERNORM) {
             const uint32_t n = layernorm_rows(c, op, it.local, widx, lane);
             WAIT_OR_RETURN(n != 0u);
             item += (n - 1u) * gridDim.x;
           } else {
-            rowwise_item(op, it.local, widx, lane, P, s);
+            embed_item(op, it.local, widx, lane, P, s);
           }
           break;
         case OP_PATCHIFY:
@@ -2358,6 +2353,7 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
       mbar_init(smem_u32(&ctrl->acc_empty[i]), kSimtWarps);
     }
     mbar_init(smem_u32(&ctrl->group_bar), kSimtWarps);
+    for (uint32_t i = 0; i < 6; ++i) mbar_init(smem_u32(&ctrl->row_bar[i]), i < 4 ? 2 : 4);
     mbar_init(smem_u32(&ctrl->cl_bar), P.cluster);
     ctrl->abort_flag = 0;
     ctrl->failure = 0;
@@ -2402,6 +2398,7 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
   c.store_stage = base + kASlots * kSlotBytes + kBSlots * kBSlotBytes + kCtrlBytes;
   c.stage = P.stage_begin;
   c.group_phase = 0;
+  c.row_phase = 0;
 
   // The launch gives every thread 168 registers (384 x 168 = 64 512). The first four warps need 72; what
   // they leave goes to the epilogue warps: 128 x 72 + 256 x 216 = 64 512.

@@ -199,12 +199,12 @@ int validate_plan(const Plan& P, std::string* err) {
       case OP_EMBED:
       case OP_ASSEMBLE:
         if (d.cols == 0 || d.cols % 4 || d.cols > 2048) return bad(n + "row length");
-        if (d.row_warps) {
-          if (d.kind != OP_LAYERNORM || (d.row_warps != 1 && d.row_warps != 2 && d.row_warps != 4) ||
-              d.cols % (4 * d.row_warps) || d.cols > d.row_warps * 512u || d.lds % 4 || d.ldo % 4 || d.ldr % 4 ||
-              (d.flags & F_NO_NORM))
+        if (d.kind == OP_LAYERNORM) {
+          if ((d.row_warps != 1 && d.row_warps != 2 && d.row_warps != 4) || d.cols > d.row_warps * 512u ||
+              (d.row_warps == 2 && d.cols <= 512) || (d.row_warps == 4 && d.cols % 16 && d.cols <= 1024) ||
+              d.lds % 4 || d.ldo % 4 || d.ldr % 4 || (d.flags & F_NO_NORM))
             return bad(n + "warps per row");
-          if ((d.flags & F_ROW_SPLIT) && d.row_warps != 4) return bad(n + "warps per row");
+          if ((d.flags & F_ROW_SPLIT) && (d.row_warps != 4 || d.cols % 16)) return bad(n + "warps per row");
           const uint32_t per_item = (d.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
           if (d.n_items != (d.rows + per_item - 1) / per_item) return bad(n + "item count");
         } else if (d.n_items != (d.rows + kRowsPerItem - 1) / kRowsPerItem) return bad(n + "item count");
@@ -966,19 +966,12 @@ int schedule(const FGraph& g, const TuningSpec& spec_in, uint32_t sm_count, Plan
           // load -> reduce -> normalise -> store chain runs on a single warp, so four warps share a row
           // when all items still fit one wave of the CTAs (BERT-base b1: 4 us of an inference). Many
           // rows: as few as the 512 columns that a warp holds allow.
-          d.row_warps = 0;
-          if (!(o.flags & F_NO_NORM)) {
-            if (spec_in.row_split != 1 && o.cols % 16 == 0 && o.cols <= 2048 &&
-                (o.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem <= P.grid) {
-              d.row_warps = 4;
-              d.flags |= F_ROW_SPLIT;
-            } else if (o.cols <= 512) {
-              d.row_warps = 1;
-            } else if (o.cols <= 1024 && o.cols % 8 == 0) {
-              d.row_warps = 2;
-            } else if (o.cols % 16 == 0) {
-              d.row_warps = 4;
-            }
+          if (spec_in.row_split != 1 && o.cols % 16 == 0 &&
+              (o.rows + kSplitRowsPerItem - 1) / kSplitRowsPerItem <= P.grid) {
+            d.row_warps = 4;
+            d.flags |= F_ROW_SPLIT;
+          } else {
+            d.row_warps = o.cols <= 512 ? 1u : o.cols <= 1024 ? 2u : 4u;
           }
           const uint32_t rows_per_item = (d.flags & F_ROW_SPLIT) ? kSplitRowsPerItem : kRowsPerItem;
           d.n_items = (o.rows + rows_per_item - 1) / rows_per_item;

@@ -101,8 +101,7 @@ struct alignas(16) OpDesc {
   uint32_t rows;            // row count for row-wise ops
   uint32_t lds;             // leading dim of row-wise source
   uint32_t vocab;           // embed: word-table rows (ids are not clamped, as in the reference)
-  uint32_t row_warps;       // LayerNorm: warps that share a row (1, 2 or 4; at most 512 columns each),
-                            // 0: one warp per row (a row length that 4 x warps does not divide)
+  uint32_t row_warps;       // LayerNorm: warps that share a row (1, 2 or 4; at most 512 columns each)
   uint32_t flag_target;     // row op that follows its producer GEMM inside one stage: arrivals to wait for
   uint32_t wait_target;     // GEMM that follows the attention it reads inside one stage: arrivals to wait for
   uint64_t p[8];
