@@ -350,9 +350,7 @@ struct Ctx {
 // the whole kernel under the calling convention: state in memory around it, and no register beyond
 // the launch's share for any role), so it only takes notes in shared memory; the notes reach the
 // status word when the role returns (publish_failure).
-__device__ __forceinline__ uint32_t coarse_time() {
-  return static_cast<uint32_t>(globaltimer_ns() >> 10);  // units of 1.024 us
-}
+__device__ __forceinline__ uint32_t coarse_time() { return wait_clock(globaltimer_ns()); }
 __device__ __forceinline__ bool give_up(const Ctx& c, uint32_t& t0, StatusCode code, uint32_t where, bool ask_others) {
   volatile uint32_t* af = &c.ctrl->abort_flag;
   if (*af) return true;
@@ -361,8 +359,8 @@ __device__ __forceinline__ bool give_up(const Ctx& c, uint32_t& t0, StatusCode c
     return true;
   }
   const uint32_t now = coarse_time();
-  if (t0 == 0u) t0 = now | 1u;  // the timer is slow and most waits end before it is read
-  if (static_cast<int32_t>(now - t0 - c.P->timeout_us) <= 0) return false;
+  if (t0 == 0u) t0 = now;  // the timer is slow and most waits end before it is read
+  if (!wait_expired(now, t0, c.P->timeout)) return false;
   atomicCAS(&c.ctrl->failure, 0ull,
             static_cast<unsigned long long>(c.stage) << 32 | static_cast<uint32_t>(code) << 16 | where);
   *af = 1;

@@ -230,7 +230,7 @@ extern "C" int mononn_attention_noalloc(const void* q, const void* k, const void
   kp.status = reinterpret_cast<KernelStatus*>(s + kOffStatus);
   kp.n_stages = 1;
   kp.epoch_base = 0;
-  kp.timeout_us = 2000000u;
+  kp.timeout = wait_ticks(2000000u);
   kp.stage_begin = 0;
   kp.stage_end = 1;
   kp.cluster = 1;

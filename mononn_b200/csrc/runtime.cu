@@ -397,7 +397,7 @@ int Runtime::launch(void* const* args, int n, void* stream, uint32_t stage_begin
   kp.hot_const_bytes = plan_.hot_const_bytes;
   kp.n_stages = static_cast<uint32_t>(plan_.stages.size());
   kp.epoch_base = epoch_;
-  kp.timeout_us = timeout_us ? timeout_us : 2000000u;
+  kp.timeout = wait_ticks(timeout_us ? timeout_us : 2000000u);
   kp.stage_begin = stage_begin;
   kp.stage_end = stage_end;
   // Arrival counters of row ops that share a stage with their GEMMs grow by the same amount on

@@ -9,6 +9,12 @@
 #pragma once
 #include <stdint.h>
 
+#ifdef __CUDACC__
+#define MONONN_HOST_DEVICE __host__ __device__
+#else
+#define MONONN_HOST_DEVICE
+#endif
+
 namespace mononn {
 
 enum OpKind : uint32_t {
@@ -143,6 +149,16 @@ enum StatusCode : uint32_t {
   ST_MBARRIER_TIMEOUT = 2,
 };
 
+// The clock of the bounded waits: the upper part of the nanosecond timer in 32 bits, in units of 2.048 us
+// and always odd, so that zero can mean "not read yet" and a later reading is never below an
+// earlier one. It comes round after 146 minutes; the longest bound, 2^32 - 1 us, is 71.6.
+// A wait gives up no earlier than its bound says, and at most 2.4 % and 13 us later.
+MONONN_HOST_DEVICE constexpr uint32_t wait_clock(uint64_t ns) { return static_cast<uint32_t>(ns >> 11) | 1u; }
+constexpr uint32_t wait_ticks(uint32_t timeout_us) { return timeout_us / 2u + (timeout_us & 1u) + 2u; }
+MONONN_HOST_DEVICE constexpr bool wait_expired(uint32_t now, uint32_t since, uint32_t ticks) {
+  return now - since > ticks;
+}
+
 // Shared-memory ring geometry (bytes).
 constexpr uint32_t kSlotBytes = 16384;   // activation ring slot: one 128x64 f16 operand tile
 constexpr uint32_t kBSlotBytes = 32768;  // weight ring slot: up to 256 rows of 64 f16 (one TMA box)
@@ -178,7 +194,7 @@ struct KernelParams {
   uint64_t hot_const_bytes;
   uint32_t n_stages;
   uint32_t epoch_base;   // counter value at kernel entry
-  uint32_t timeout_us;   // bound on every wait
+  uint32_t timeout;      // bound on every wait: wait_ticks(microseconds)
   uint32_t stage_begin;  // run stages [stage_begin, stage_end)
   uint32_t stage_end;
   uint32_t cluster;      // CTAs per cluster of this launch (1: no cluster-scoped arrival)
