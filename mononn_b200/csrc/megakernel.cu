@@ -145,11 +145,12 @@ __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((sadd
 // descriptors assembled in 64 bits a k block of a 64-column tile took 0.30 us, this way 0.20; see
 // also the loop in role_mma.
 __device__ __forceinline__ void mma_kblock(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                           uint32_t accumulate, uint32_t a_empty, uint32_t b_empty, bool free_b) {
+                                           uint32_t accumulate, uint32_t a_empty, uint32_t b_empty, bool free_b,
+                                           bool issuer) {
   asm volatile(
       "{\n\t.reg .pred q, p, f, w;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t.reg .b32 t;\n\t"
       "setp.eq.u32 w, 0, 0;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.u32 q, %9, 0;\n\t"
       "setp.ne.u32 p, %4, 0;\n\t"
       "setp.ne.and.u32 f, %7, 0, q;\n\t"
       "mov.b64 a0, {%1, %8};\n\tmov.b64 b0, {%2, %8};\n\t"
@@ -164,7 +165,7 @@ __device__ __forceinline__ void mma_kblock(uint32_t tmem_d, uint32_t a_lo, uint3
       "@f tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
       "}" ::"r"(tmem_d),
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(a_empty), "r"(b_empty),
-      "r"(static_cast<uint32_t>(free_b)), "r"(kDescHi)
+      "r"(static_cast<uint32_t>(free_b)), "r"(kDescHi), "r"(static_cast<uint32_t>(issuer))
       : "memory");
 }
 // One lane of a converged warp (the same one every time for a full mask).
@@ -509,6 +510,22 @@ __device__ __forceinline__ bool group_sync(Ctx& c, uint32_t where) {
     if (!(expr)) return;     \
   } while (0)
 
+// The roles of the first warps run all lanes alike and poll their barriers with all of them, without a
+// vote in each wait (that took 2 to 5 % of an inference). So that no lane is waited for without a
+// bound should some give up a wait that others saw end: all their warp-wide instructions between two
+// waits are votes with the same mask, one for each stage and item and one at the end. A lane that gives up casts its
+// `false` once on leaving the role, which is what the others' next vote meets; a vote that fails takes
+// everybody out. (Nothing in a k block is warp-wide: the lane that issues is chosen once.)
+#define WAIT_OR_LEAVE(expr)    \
+  do {                         \
+    if (!(expr)) return false; \
+  } while (0)
+#define VOTE_OR_RETURN(expr)  \
+  do {                        \
+    if (!(expr)) return true; \
+  } while (0)
+__device__ __forceinline__ bool all_here() { return __all_sync(0xffffffffu, true); }
+
 struct Item {
   const OpDesc* op;
   uint32_t local;  // item index inside the op
@@ -622,7 +639,7 @@ __device__ __forceinline__ void tma_issue(bool issuer, bool hint, uint32_t dst, 
 // Role: weight producer (warp 0). Like the MMA role, the producers run all 32 lanes converged
 // and one elected lane issues the copies and the barrier arrivals.
 // ----------------------------------------------------------------------------
-__device__ void role_weight_producer(Ctx c, uint32_t lane) {
+__device__ __forceinline__ bool role_weight_producer(Ctx c, uint32_t lane) {
   const KernelParams& P = *c.P;
   const bool issuer = elect_one_sync();
   const uint8_t* tmaps = static_cast<const uint8_t*>(P.tmaps);
@@ -631,6 +648,7 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
   uint32_t b_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
+    VOTE_OR_RETURN(all_here());
     const StageDesc& st = load_stage(P, c.ctrl, 0u, s, lane);
     {
       // If the stage holds attention items that compute their own projections, only a few SMs will
@@ -656,6 +674,7 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
       }
     }
     for (uint32_t item = blockIdx.x; item < st.n_items; item += gridDim.x) {
+      VOTE_OR_RETURN(all_here());
       const Item it = fetch_item<true>(P, st, item, c.ctrl->desc[0], lane);
       const OpDesc& op = *it.op;
       if (op.kind == OP_ATTENTION && attn_fused(op)) {
@@ -667,7 +686,7 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
                               tmaps + static_cast<size_t>(op.vocab) * 128u};
         for (uint32_t kb = 0; kb < nkb; ++kb) {
           const uint32_t slot = b_cnt % kBSlots, use = b_cnt / kBSlots;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->b_empty[slot], (use & 1u) ^ 1u, 0x101));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->b_empty[slot], (use & 1u) ^ 1u, 0x101));
           const uint32_t full = smem_u32(&c.ctrl->b_full[slot]);
           if (issuer) mbar_arrive_expect_tx(full, 3u * 8192u);
 #pragma unroll
@@ -692,7 +711,7 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
         const uint32_t kb = grp * kbps;  // ((gi + rot) % groups) * kbps
         if (++grp == groups) grp = 0;
         const uint32_t slot = b_cnt % kBSlots, use = b_cnt / kBSlots;
-        WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->b_empty[slot], (use & 1u) ^ 1u, 0x100));
+        WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->b_empty[slot], (use & 1u) ^ 1u, 0x100));
         const uint32_t full = smem_u32(&c.ctrl->b_full[slot]);
         if (issuer) mbar_arrive_expect_tx(full, bytes);
         tma_issue(issuer, hint, c.b_ring + slot * kBSlotBytes, tm, 0, static_cast<int32_t>(row0 + kb * op.n_tile),
@@ -702,12 +721,14 @@ __device__ void role_weight_producer(Ctx c, uint32_t lane) {
       if (issuer) trace(P, s, TR_W_ISSUED);
     }
   }
+  VOTE_OR_RETURN(all_here());
+  return true;
 }
 
 // ----------------------------------------------------------------------------
 // Role: activation producer (warp 1)
 // ----------------------------------------------------------------------------
-__device__ void role_act_producer(Ctx c, uint32_t lane) {
+__device__ __forceinline__ bool role_act_producer(Ctx c, uint32_t lane) {
   const KernelParams& P = *c.P;
   const bool issuer = elect_one_sync();
   const uint8_t* tmaps = static_cast<const uint8_t*>(P.tmaps);
@@ -716,6 +737,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
   uint32_t a_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
+    VOTE_OR_RETURN(all_here());
     const StageDesc& st = load_stage(P, c.ctrl, 1u, s, lane);
     Item first{nullptr, 0};
     if (blockIdx.x < st.n_items) {
@@ -731,6 +753,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
     }
     bool waited = false;
     for (uint32_t item = blockIdx.x; item < st.n_items; item += gridDim.x) {
+      VOTE_OR_RETURN(all_here());
       const Item it = (item == blockIdx.x) ? first : fetch_item<true>(P, st, item, c.ctrl->desc[1], lane);
       const OpDesc& op = *it.op;
       if (op.kind != OP_GEMM && op.kind != OP_ATTENTION) continue;
@@ -745,7 +768,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
       if (!waited) {
         bool ok = true;  // one lane polls the global counter; the acquire, the proxy fence and the copies are its
         if (issuer) ok = grid_wait(c, s, 0x200, false);
-        WAIT_OR_RETURN(__all_sync(0xffffffffu, ok));
+        VOTE_OR_RETURN(__all_sync(0xffffffffu, ok));
         fence_proxy_async_global();
         waited = true;
         if (issuer) trace(P, s, TR_ACT_READY);
@@ -755,7 +778,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
           // the A operand is the output of an attention operator of this stage: wait until all of
           // its items have counted themselves (each after its stores, with release), then make
           // those stores visible to the copies as after a grid barrier
-          WAIT_OR_RETURN(flag_wait_warp(c, op.wait_flag, op.wait_target, 0x204));
+          VOTE_OR_RETURN(flag_wait_warp(c, op.wait_flag, op.wait_target, 0x204));
           fence_proxy_async_global();
           if (issuer) trace(P, s, TR_MARK0 + 7);
         }
@@ -771,7 +794,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
             if (++grp == groups) grp = 0;
           }
           const uint32_t slot = a_cnt % kASlots, use = a_cnt / kASlots;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x201));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x201));
           const uint32_t full = smem_u32(&c.ctrl->a_full[slot]);
           if (issuer) mbar_arrive_expect_tx(full, kSlotBytes);
           tma_issue(issuer, hint, c.a_ring + slot * kSlotBytes, tm, static_cast<int32_t>((t.ks * nkb + kb) * 64u),
@@ -788,7 +811,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
           // the k-block tiles of this batch's rows of x; Q, K, V^T and P are written on chip
           for (uint32_t kb = 0; kb < op.kb_per_split; ++kb) {
             const uint32_t slot = a_cnt % kASlots, use = a_cnt / kASlots;
-            WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x203));
+            WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x203));
             const uint32_t full = smem_u32(&c.ctrl->a_full[slot]);
             if (issuer) mbar_arrive_expect_tx(full, kSlotBytes);
             tma_issue(issuer, false, c.a_ring + slot * kSlotBytes, tm, static_cast<int32_t>(kb * 64u),
@@ -803,7 +826,7 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
         for (uint32_t j = 0; j < 1u + 2u * nc; ++j) {
           if (j > nc) a_cnt += (j == nc + 1u) ? 0u : 2u;  // step over the previous chunk's P slots
           const uint32_t slot = a_cnt % kASlots, use = a_cnt / kASlots;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x202));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_empty[slot], (use & 1u) ^ 1u, 0x202));
           const uint32_t full = smem_u32(&c.ctrl->a_full[slot]);
           const uint32_t dst = c.a_ring + slot * kSlotBytes;
           if (issuer) mbar_arrive_expect_tx(full, kSlotBytes);
@@ -826,6 +849,8 @@ __device__ void role_act_producer(Ctx c, uint32_t lane) {
       if (issuer) trace(P, s, TR_ACT_ISSUED);
     }
   }
+  VOTE_OR_RETURN(all_here());
+  return true;
 }
 
 // The MMA issuer's place in the two rings, kept as slot and parity (a count would be divided by the
@@ -869,21 +894,23 @@ struct MmaRing {
 // a loop of four instructions, a commit and a wait per k block measured 88 cycles per
 // instruction this way against 121 when a single lane ran it (probe: mononn_debug_mma_issue).
 // ----------------------------------------------------------------------------
-__device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
+__device__ __forceinline__ bool role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
   const KernelParams& P = *c.P;
   const bool issuer = elect_one_sync();
   MmaRing ring(c);
   uint32_t acc_cnt = 0;
   for (uint32_t s = P.stage_begin; s < P.stage_end; ++s) {
     c.stage = s;
+    VOTE_OR_RETURN(all_here());
     const StageDesc& st = load_stage(P, c.ctrl, 2u, s, lane);
     for (uint32_t item = blockIdx.x; item < st.n_items; item += gridDim.x) {
+      VOTE_OR_RETURN(all_here());
       const Item it = fetch_item<true>(P, st, item, c.ctrl->desc[2], lane);
       const OpDesc& op = *it.op;
       if (op.kind == OP_GEMM) {
         const uint32_t nkb = op.kb_per_split, kbps = op.kb_per_bslot;
         const uint32_t buf = acc_cnt & 1u;
-        WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[buf], ((acc_cnt >> 1) & 1u) ^ 1u, 0x300));
+        WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->acc_empty[buf], ((acc_cnt >> 1) & 1u) ^ 1u, 0x300));
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * kAccCols;
         const uint32_t idesc = umma_idesc_m128(op.n_tile);
@@ -892,10 +919,10 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         uint32_t a_rdy = ring.a_peek(), b_rdy = ring.b_peek();
         for (uint32_t kb = 0; kb < nkb; ++kb) {
           if (sub == 0) {
-            if (!b_rdy) WAIT_OR_RETURN(ring.b_wait(c, 0x301));
+            if (!b_rdy) WAIT_OR_LEAVE(ring.b_wait(c, 0x301));
             b_lo = ring.b_lo();
           }
-          if (!a_rdy) WAIT_OR_RETURN(ring.a_wait(c, 0x302));
+          if (!a_rdy) WAIT_OR_LEAVE(ring.a_wait(c, 0x302));
           if (kb == 0) if (issuer) trace(P, s, TR_MMA_FIRST);
           const uint32_t a_lo = ring.a_lo(), a_empty = ring.a_empty(), b_empty = ring.b_empty();
           const bool last_sub = (++sub == kbps) || kb + 1u == nkb;
@@ -909,7 +936,7 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
           a_rdy = ring.a_peek();
           b_rdy = ring.b_peek();
           tc_fence_after();
-          mma_kblock(tmem_d, a_lo, b_lo, idesc, kb, a_empty, b_empty, last_sub);
+          mma_kblock(tmem_d, a_lo, b_lo, idesc, kb, a_empty, b_empty, last_sub, issuer);
           b_lo += sub_step;
         }
         if (issuer) tc_commit(smem_u32(&c.ctrl->acc_full[buf]));
@@ -924,14 +951,14 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         if (attn_fused(op)) {
           // [Q_h | K_h | V_h] = x_b W_h into 192 columns; the accumulator overlaps both GEMM buffers
           const uint32_t phQ = ph++, nkb = op.kb_per_split;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[phQ & 1u], ((phQ >> 1) & 1u) ^ 1u, 0x320));
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[ph & 1u], ((ph >> 1) & 1u) ^ 1u, 0x321));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->acc_empty[phQ & 1u], ((phQ >> 1) & 1u) ^ 1u, 0x320));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->acc_empty[ph & 1u], ((ph >> 1) & 1u) ^ 1u, 0x321));
           tc_fence_after();
           const uint32_t idesc = umma_idesc_m128(192);
           uint32_t a_rdy = ring.a_peek(), b_rdy = ring.b_peek();
           for (uint32_t kb = 0; kb < nkb; ++kb) {
-            if (!b_rdy) WAIT_OR_RETURN(ring.b_wait(c, 0x322));
-            if (!a_rdy) WAIT_OR_RETURN(ring.a_wait(c, 0x323));
+            if (!b_rdy) WAIT_OR_LEAVE(ring.b_wait(c, 0x322));
+            if (!a_rdy) WAIT_OR_LEAVE(ring.a_wait(c, 0x323));
             if (kb == 0) if (issuer) trace(P, s, TR_MMA_FIRST);
             const uint32_t a_lo = ring.a_lo(), b_lo = ring.b_lo(), a_empty = ring.a_empty(), b_empty = ring.b_empty();
             ring.a_next();
@@ -939,7 +966,7 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
             a_rdy = ring.a_peek();
             b_rdy = ring.b_peek();
             tc_fence_after();
-            mma_kblock(tmem_base + kAttnQkvCol, a_lo, b_lo, idesc, kb, a_empty, b_empty, true);
+            mma_kblock(tmem_base + kAttnQkvCol, a_lo, b_lo, idesc, kb, a_empty, b_empty, true, issuer);
           }
           if (issuer) tc_commit(smem_u32(&c.ctrl->acc_full[phQ & 1u]));
           if (issuer) trace(P, s, TR_MMA_LAST);
@@ -947,13 +974,13 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         }
         // the scores may span both accumulator buffers: both must have been drained
         const uint32_t phS = ph, phO = ph + 1u;
-        WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[phS & 1u], ((phS >> 1) & 1u) ^ 1u, 0x310));
-        WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->acc_empty[phO & 1u], ((phO >> 1) & 1u) ^ 1u, 0x313));
+        WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->acc_empty[phS & 1u], ((phS >> 1) & 1u) ^ 1u, 0x310));
+        WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->acc_empty[phO & 1u], ((phO >> 1) & 1u) ^ 1u, 0x313));
         // S_j = Q K_j^T  (128 x 128, K = 64) into columns j*128
-        WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(base)], par_of(base), 0x311));
+        WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_full[slot_of(base)], par_of(base), 0x311));
         for (uint32_t j = 0; j < nc; ++j) {
           const uint32_t kc = base + 1u + j;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(kc)], par_of(kc), 0x312));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_full[slot_of(kc)], par_of(kc), 0x312));
           tc_fence_after();
           const uint64_t ad = umma_desc_sw128(c.a_ring + slot_of(base) * kSlotBytes);
           const uint64_t bd = umma_desc_sw128(c.a_ring + slot_of(kc) * kSlotBytes);
@@ -968,9 +995,9 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
         // O += P_j V_j  (128 x 64, K = 128 per chunk) into columns kAttnOutCol..
         for (uint32_t j = 0; j < nc; ++j) {
           const uint32_t vc = base + 1u + nc + 3u * j;
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(vc)], par_of(vc), 0x314));
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(vc + 1u)], par_of(vc + 1u), 0x315));
-          WAIT_OR_RETURN(mbar_wait(c, &c.ctrl->a_full[slot_of(vc + 2u)], par_of(vc + 2u), 0x316));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_full[slot_of(vc)], par_of(vc), 0x314));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_full[slot_of(vc + 1u)], par_of(vc + 1u), 0x315));
+          WAIT_OR_LEAVE(mbar_wait(c, &c.ctrl->a_full[slot_of(vc + 2u)], par_of(vc + 2u), 0x316));
           tc_fence_after();
           const uint32_t idesc = umma_idesc_m128(64);
 #pragma unroll
@@ -989,6 +1016,8 @@ __device__ void role_mma(Ctx c, uint32_t tmem_base, uint32_t lane) {
       }
     }
   }
+  VOTE_OR_RETURN(all_here());
+  return true;
 }
 
 // ----------------------------------------------------------------------------
@@ -2402,9 +2431,11 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
   // they leave goes to the epilogue warps: 128 x 72 + 256 x 216 = 64 512.
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    if (warp == 0) role_weight_producer(c, lane);
-    else if (warp == 1) role_act_producer(c, lane);
-    else if (warp == 2) role_mma(c, tmem_base, lane);
+    bool voted = true;  // false: this lane gave up a wait, and the other lanes have yet to hear of it
+    if (warp == 0) voted = role_weight_producer(c, lane);
+    else if (warp == 1) voted = role_act_producer(c, lane);
+    else if (warp == 2) voted = role_mma(c, tmem_base, lane);
+    if (!voted) __all_sync(0xffffffffu, false);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     role_simt(c, tmem_base, threadIdx.x - kRoleThreads);
