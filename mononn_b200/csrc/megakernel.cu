@@ -2428,16 +2428,17 @@ mononn_megakernel(const __grid_constant__ KernelParams P) {
   c.row_phase = 0;
 
   // The launch gives every thread 168 registers (384 x 168 = 64 512). The first four warps need 72; what
-  // they leave goes to the epilogue warps: 128 x 72 + 256 x 216 = 64 512.
+  // they leave goes to the epilogue warps: 128 x 72 + 256 x 216 = 64 512. (The host checks that the
+  // kernel was built with as many before it launches it: register_split_fits.)
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
     bool voted = true;  // false: this lane gave up a wait, and the other lanes have yet to hear of it
     if (warp == 0) voted = role_weight_producer(c, lane);
     else if (warp == 1) voted = role_act_producer(c, lane);
     else if (warp == 2) voted = role_mma(c, tmem_base, lane);
     if (!voted) __all_sync(0xffffffffu, false);
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSimtRegs));
     role_simt(c, tmem_base, threadIdx.x - kRoleThreads);
   }
   __syncwarp();

@@ -89,6 +89,10 @@ int setup(int dev, DeviceState** out) {
     void* p = nullptr;
     NA_TRY(cudaGetSymbolAddress(&p, g_noalloc_scratch));
     if (p == nullptr) return fail(MONONN_ERR_CUDA, "cudaGetSymbolAddress returned a null address");
+    cudaFuncAttributes fa;
+    NA_TRY(cudaFuncGetAttributes(&fa, mononn_megakernel));
+    if (!register_split_fits(fa.numRegs))
+      return fail(MONONN_ERR_CUDA, "the kernel was built with fewer registers than its warps share out");
     NA_TRY(cudaFuncSetAttribute(mononn_megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kSmemBytes)));
     if (g_encode == nullptr) {

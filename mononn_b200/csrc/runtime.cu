@@ -102,6 +102,13 @@ int Runtime::init(int device) {
     set_last_error("cuTensorMapEncodeTiled is not available from the driver");
     return MONONN_ERR_CUDA;
   }
+  cudaFuncAttributes fa;
+  CUDA_TRY(cudaFuncGetAttributes(&fa, mononn_megakernel));
+  if (!register_split_fits(fa.numRegs)) {
+    set_last_error("the kernel was built with " + std::to_string(fa.numRegs) +
+                   " registers a thread, fewer than its warps share out");
+    return MONONN_ERR_CUDA;
+  }
   CUDA_TRY(cudaFuncSetAttribute(mononn_megakernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kSmemBytes)));
   attr_set_ = true;

@@ -176,6 +176,15 @@ constexpr uint32_t kRoleThreads = 128;        // warps 0..3: producers and the M
 constexpr uint32_t kSimtThreads = 256;        // warps 4..11: epilogue / row-wise work
 constexpr uint32_t kSimtWarps = kSimtThreads / 32;
 constexpr uint32_t kThreads = kRoleThreads + kSimtThreads;
+// Registers a thread, moved from the role warps to the epilogue warps at kernel start (setmaxnreg). The
+// sum has to fit what the launch gives all threads: taking more than is there would wait for ever.
+constexpr uint32_t kRoleRegs = 72;
+constexpr uint32_t kSimtRegs = 216;
+constexpr bool register_split_fits(int regs_per_thread) {
+  return regs_per_thread > 0 &&
+         kThreads * static_cast<uint32_t>(regs_per_thread) >= kRoleThreads * kRoleRegs + kSimtThreads * kSimtRegs;
+}
+static_assert(kRoleRegs % 8 == 0 && kSimtRegs % 8 == 0 && kSimtRegs <= 256, "setmaxnreg takes multiples of 8");
 constexpr uint32_t kRowsPerItem = kSimtWarps;  // row-wise operators: one row per SIMT warp per work item
 constexpr uint32_t kSplitRowsPerItem = 2;      // LayerNorm with F_ROW_SPLIT
 constexpr uint32_t kTmemCols = 512;
