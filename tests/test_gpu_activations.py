@@ -28,15 +28,16 @@ def run_with_bias(act, value):
         return got, R.bert_encoder(cfg, w, inp)
 
 
+@pytest.mark.parametrize("act", ["gelu_erf", "quick_gelu", "gelu_tanh"])
 @pytest.mark.parametrize("value", [math.nan, math.inf, -math.inf], ids=str)
-def test_gelu_passes_on_what_is_not_finite(value):
-    """gelu(NaN) and gelu(-inf) = -inf * 0 are NaN, gelu(inf) is inf: each reaches every column of every
-    row through FFN-down and the norm behind it."""
-    got, want = run_with_bias("gelu_erf", value)
+def test_what_is_not_finite_is_passed_on(act, value):
+    """f(NaN) and f(-inf) = -inf * 0 are NaN, f(inf) is inf: each reaches every column of every row through
+    FFN-down and the norm behind it."""
+    got, want = run_with_bias(act, value)
     assert np.isnan(want).all() and np.isnan(got).all()
 
 
-@pytest.mark.parametrize("act", ["gelu_erf", "quick_gelu"])
+@pytest.mark.parametrize("act", ["gelu_erf", "quick_gelu", "gelu_tanh"])
 @pytest.mark.parametrize("value", [3e4, -3e4], ids=str)
 def test_activations_of_large_values(act, value):
     got, want = run_with_bias(act, value)
