@@ -390,7 +390,7 @@ __device__ __forceinline__ void publish_failure(const KernelParams& P, Ctrl* ctr
   }
 }
 
-// Optional per-CTA event trace: trace[(cta * n_stages + stage) * 8 + event] = %globaltimer.
+// Optional per-CTA event trace: trace[(cta * n_stages + stage) * kTraceEvents + event] = %globaltimer.
 enum TraceEvent : uint32_t {
   TR_SIMT_READY = 0,   // epilogue warps passed the previous stage's grid barrier
   TR_SIMT_DONE = 1,    // ... finished this stage's items
@@ -1021,9 +1021,10 @@ __device__ __forceinline__ bool role_mma(Ctx c, uint32_t tmem_base, uint32_t lan
 }
 
 // ----------------------------------------------------------------------------
-// Epilogue / SIMT math. Everything here runs once per stage on four warps, so the code
-// is kept compact (chunk loops are not unrolled, slow paths are out of line): the whole
-// kernel has to stay resident in the instruction cache across a layer's stages.
+// Epilogue / SIMT math. Everything here runs once per stage on eight warps, so the code is kept
+// compact (chunk loops are not unrolled, one instance of each kind of work): the kernel's instructions
+// compete for the instruction cache across a layer's stages. All of it is inline: a call would put
+// the kernel under the calling convention (see bounded_wait).
 // ----------------------------------------------------------------------------
 // Two f32 operations in one instruction (the packed forms of sm_100).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -2198,10 +2199,12 @@ __device__ __forceinline__ bool attention_simt(Ctx& c, const OpDesc& op, uint32_
 // ----------------------------------------------------------------------------
 // Role: epilogue + SIMT stages + grid barrier (warps 4..11)
 //
-// The whole kernel is some 210 KB of instructions, of which a layer runs about half, and the instruction
+// The whole kernel is some 219 KB of instructions, of which a layer runs about half, and the instruction
 // cache is what a stage's first pass through each part pays for: code that nothing in a graph runs
 // still costs it (24 KB of it made BERT-base b1 3 % slower, 41 KB 5.5 %, all sizes alike). So each
-// kind of work has one instance of its code here, also where a second one would take fewer instructions.
+// kind of work has one instance of its code here (norms: NormRows; rows of an embedding: embed_item),
+// also where a second one would take fewer instructions. A few KB more or less no longer show; how
+// the code happens to lie does (BERT-base b1 436 or 447 us).
 // ----------------------------------------------------------------------------
 __device__ void role_simt(Ctx c, uint32_t tmem_base, uint32_t tid_in_group) {
   const KernelParams& P = *c.P;
