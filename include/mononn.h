@@ -50,7 +50,7 @@ typedef struct {
   int tuning_level;             /* what mononn_tune searches: 0 nothing (times the heuristic spec),
                                    1 stage structure (qkv_fusion, row_fusion) and per-GEMM-class
                                    tiles timed on their own stage, 2 + the number of CTAs */
-  unsigned barrier_timeout_us;  /* bound on every in-kernel wait; 0 = 2 000 000 */
+  unsigned barrier_timeout_us;  /* bound on every in-kernel wait, any value up to 2^32 - 1; 0 = 2 000 000 */
 } mononn_options;
 
 typedef struct {
